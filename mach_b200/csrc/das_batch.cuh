@@ -58,7 +58,7 @@ __device__ __forceinline__ void copy_words(T* dst, const T* src) {
 }
 
 template <int S, int INTERP, int NF, bool SPLIT, int CS = 1>
-__global__ void __launch_bounds__(kLaneVoxelThreads, NF == 16 ? 4 : 8)
+__global__ void __launch_bounds__(kLaneVoxelThreads, lane_voxel_ctas<S, INTERP, NF>() - (NF >= 8 ? 1 : 0))
     das_lane_voxel_persistent(const BatchHeader* __restrict__ hdr, const BatchJob* __restrict__ jobs,
                               const int64_t* __restrict__ item_begin, unsigned long long* counter) {
     extern __shared__ float smem_words[];

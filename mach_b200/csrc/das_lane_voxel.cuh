@@ -92,24 +92,38 @@ __device__ __forceinline__ void split_phasor(float cycles, float& sn, float& cs)
     __sincosf(__fmul_rn(__fsub_rn(cycles, whole), 6.28318530717958647f), &sn, &cs);
 }
 
-// Interpolated sample at `row[idx * stride]` (stride = frames), widened to FP32.  PACKED:
-// complex quadratic taps in packed FP32x2, the same operations and order as the scalar form.
+// One int16 sample as float without the conversion pipe (see widen_i16x2): x + 32768 in the
+// mantissa of 2^23, minus 2^23 + 32768, exact.
+template <int S>
+__device__ __forceinline__ float2 load_sample(const typename Storage<S>::T* p) {
+    if constexpr (S == kI16) {
+        const unsigned u = __ldg(reinterpret_cast<const unsigned short*>(p));
+        return make_float2(__fsub_rn(__uint_as_float(u ^ 0x4B008000u), 8421376.0f), 0.f);
+    } else {
+        return Storage<S>::load(p);
+    }
+}
+
+// Interpolated sample from tap 0 at `p` (linear: second tap at `p1`; quadratic: taps `stride`
+// samples around `p`), widened to FP32.  PACKED: complex quadratic taps in packed FP32x2, the
+// same operations and order as the scalar form.
 template <int S, int INTERP, bool PACKED = false>
-__device__ __forceinline__ float2 tap_value(const typename Storage<S>::T* p, const TapPosition& tp, int stride) {
+__device__ __forceinline__ float2 tap_value(const typename Storage<S>::T* p, const typename Storage<S>::T* p1,
+                                            const TapPosition& tp, int stride) {
     using ST = Storage<S>;
     if constexpr (INTERP == kNearest) {
-        return ST::load(p);
+        return load_sample<S>(p);
     } else if constexpr (INTERP == kLinear) {
-        const float2 a = ST::load(p);
-        const float2 b = ST::load(p + tp.step * stride);
+        const float2 a = load_sample<S>(p);
+        const float2 b = load_sample<S>(p1);
         float2 r;
         r.x = __fmaf_rn(tp.w0, __fsub_rn(b.x, a.x), a.x);  // a + t (b - a), mach's lerp form
         r.y = ST::kComplex ? __fmaf_rn(tp.w0, __fsub_rn(b.y, a.y), a.y) : 0.f;
         return r;
     } else {
-        const float2 a = ST::load(p - stride);
-        const float2 b = ST::load(p);
-        const float2 c = ST::load(p + stride);
+        const float2 a = load_sample<S>(p - stride);
+        const float2 b = load_sample<S>(p);
+        const float2 c = load_sample<S>(p + stride);
         if constexpr (PACKED && ST::kComplex) {
             return __ffma2_rn(make_float2(tp.w2, tp.w2), c,
                               __ffma2_rn(make_float2(tp.w0, tp.w0), a, __fmul2_rn(make_float2(tp.w1, tp.w1), b)));
@@ -297,12 +311,165 @@ __device__ __forceinline__ int64_t lane_voxel_index(const DasArgs& a, int64_t ti
     return (o < a.map_outer && f < a.map_fast) ? o * a.map_fast + f : a.n_vox;
 }
 
+// min / max that return NaN when either operand is one (a NaN arrival must fail the range test).
+__device__ __forceinline__ float min_nan(float x, float y) {
+    float r;
+    asm("min.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
+}
+__device__ __forceinline__ float max_nan(float x, float y) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(x), "f"(y));
+    return r;
+}
+
+// Smallest and largest transmit part of a voxel over the transmits of one pass (reference mode:
+// arrival times; split mode: integer sample bases).
+template <bool SPLIT>
+struct TxRange {
+    float lo = INFINITY, hi = -INFINITY;
+    __device__ __forceinline__ void add(float arrival, int) {
+        lo = min_nan(lo, arrival);
+        hi = max_nan(hi, arrival);
+    }
+    __device__ __forceinline__ void merge(int off) {  // with the lane `off` away
+        lo = min_nan(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+        hi = max_nan(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+    }
+};
+template <>
+struct TxRange<true> {
+    int lo = 0x7fffffff, hi = -0x7fffffff;
+    __device__ __forceinline__ void add(float, int base) {
+        lo = min(lo, base);
+        hi = max(hi, base);
+    }
+    __device__ __forceinline__ void merge(int off) {
+        lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, off));
+        hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, off));
+    }
+};
+
+// Whether every transmit of the pass has its taps inside the row and tau >= 0, so that the
+// transmit loop needs no test per point.  Reference mode: tau, tau - t0 and s are each a rounded
+// monotone function of the arrival, so testing the two extreme arrivals decides for all of them
+// exactly (a NaN distance or arrival fails).  Split mode: the integer bases with one sample of
+// slack for the carry of the fractions, both parts far from int overflow.  Conservative at the
+// last sample of a row (a point there takes the loop with tests), so that linear taps may read
+// idx + 1 of any storage.
+template <int INTERP, bool SPLIT>
+__device__ __forceinline__ bool taps_always_inside(const DasArgs& a, const TxRange<SPLIT>& r, float dist,
+                                                   const SplitPos& rx) {
+    if constexpr (SPLIT) {
+        constexpr int kFar = 1 << 24;
+        if (r.lo < -kFar || r.hi > kFar || static_cast<unsigned>(rx.base) > static_cast<unsigned>(kFar)) return false;
+        const int lo = r.lo + rx.base, hi = r.hi + rx.base + 1;
+        constexpr int kFirst = INTERP == kQuadratic ? 1 : 0;
+        constexpr int kLast = INTERP == kQuadratic ? 3 : (INTERP == kLinear ? 2 : 2);
+        return lo >= kFirst && lo > a.start_base && hi <= a.n_samples - kLast;
+    } else {
+        const float t_lo = __fmaf_rn(dist, a.inv_c, r.lo), t_hi = __fmaf_rn(dist, a.inv_c, r.hi);
+        const float s_lo = __fmul_rn(__fsub_rn(t_lo, a.t0), a.fs), s_hi = __fmul_rn(__fsub_rn(t_hi, a.t0), a.fs);
+        const float first = INTERP == kNearest ? -0.5f : (INTERP == kLinear ? 0.0f : 1.0f);
+        const float last = INTERP == kNearest ? a.hi_nearest : (INTERP == kLinear ? a.hi_linear : a.hi_quadratic);
+        return t_lo >= 0.0f && t_hi >= 0.0f && s_lo >= first && s_hi >= first && s_lo < last && s_hi < last;
+    }
+}
+
+// A point whose taps are known to be inside its row: byte addresses of tap 0 (quadratic: the
+// centre tap) and of the second linear tap, interpolation weights, weighted phasor.
+struct SafePoint {
+    const char* p0;
+    const char* p1;
+    TapPosition tp;
+    float cw, sw;
+};
+
+// Row address from which safe_point counts: in reference mode the integer part of the sample
+// position is used as the bits of s + 1.5 * 2^23, so the constant is taken off the row once.
+template <bool SPLIT>
+__device__ __forceinline__ const char* safe_row(const void* row, int64_t sample_bytes) {
+    return static_cast<const char*>(row) - (SPLIT ? 0 : static_cast<int64_t>(kRoundMagicBits) * sample_bytes);
+}
+
+// Position, weights and phasor of one point without range tests; the same arithmetic as
+// tap_position / split_tap_position, the second linear tap from the sample position rounded up
+// (equal to the first one when the fraction is 0, as mach's ceil).  NEXT: the second tap is always
+// the next sample, for integer samples: with a fraction of 0 it gets weight 0, which floating
+// storage cannot afford (0 times an infinity).
+template <int INTERP, bool SPLIT, bool CPLX, bool NEXT>
+__device__ __forceinline__ SafePoint safe_point(const DasArgs& a, const char* row, unsigned sample_bytes, float dist,
+                                                const SplitPos& rx_pos, float rx_cyc, float w, float arrival,
+                                                int tx_base, float tx_cyc) {
+    SafePoint q{};
+    q.cw = w;
+    if constexpr (SPLIT) {
+        int base = tx_base + rx_pos.base;
+        float frac = __fadd_rn(arrival, rx_pos.frac);
+        if (frac >= 1.0f) {
+            frac = __fsub_rn(frac, 1.0f);
+            base += 1;
+        }
+        if constexpr (INTERP == kLinear) {
+            q.tp.w0 = frac;
+            q.p0 = row + static_cast<uint64_t>(static_cast<unsigned>(base)) * sample_bytes;
+            q.p1 = q.p0 + (NEXT || frac > 0.0f ? sample_bytes : 0u);
+        } else {
+            const int up = (frac > 0.5f || (frac == 0.5f && (base & 1))) ? 1 : 0;
+            q.p0 = row + static_cast<uint64_t>(static_cast<unsigned>(base + up)) * sample_bytes;
+            if constexpr (INTERP == kQuadratic) {
+                const float x = __fsub_rn(frac, static_cast<float>(up));  // exact
+                const float hx = __fmul_rn(0.5f, x);
+                const float qq = __fmul_rn(hx, x);
+                q.tp.w0 = __fsub_rn(qq, hx);
+                q.tp.w1 = __fmaf_rn(-2.0f, qq, 1.0f);
+                q.tp.w2 = __fadd_rn(qq, hx);
+            }
+        }
+        if (CPLX && a.rotate) {
+            float sn, cs;
+            split_phasor(__fadd_rn(tx_cyc, rx_cyc), sn, cs);
+            q.cw = __fmul_rn(cs, w);
+            q.sw = __fmul_rn(sn, w);
+        }
+    } else {
+        const float tau = __fmaf_rn(dist, a.inv_c, arrival);
+        const float s = __fmul_rn(__fsub_rn(tau, a.t0), a.fs);
+        if constexpr (INTERP == kLinear) {
+            const float lo = __fadd_rd(s, kRoundMagic);
+            q.tp.w0 = __fsub_rn(s, __fsub_rn(lo, kRoundMagic));
+            q.p0 = row + static_cast<uint64_t>(__float_as_uint(lo)) * sample_bytes;
+            q.p1 = NEXT ? q.p0 + sample_bytes
+                        : row + static_cast<uint64_t>(__float_as_uint(__fadd_ru(s, kRoundMagic))) * sample_bytes;
+        } else {
+            const float r = __fadd_rn(s, kRoundMagic);
+            q.p0 = row + static_cast<uint64_t>(__float_as_uint(r)) * sample_bytes;
+            if constexpr (INTERP == kQuadratic) {
+                const float x = __fsub_rn(s, __fsub_rn(r, kRoundMagic));
+                const float hx = __fmul_rn(0.5f, x);
+                const float qq = __fmul_rn(hx, x);
+                q.tp.w0 = __fsub_rn(qq, hx);              // x (x - 1) / 2
+                q.tp.w1 = __fmaf_rn(-2.0f, qq, 1.0f);     // (1 - x)(1 + x)
+                q.tp.w2 = __fadd_rn(qq, hx);              // x (x + 1) / 2
+            }
+        }
+        if (CPLX && a.rotate) {
+            float sn, cs;
+            __sincosf(__fmul_rn(a.mod_rad, tau), &sn, &cs);  // kernel.cu:656-658
+            q.cw = __fmul_rn(cs, w);
+            q.sw = __fmul_rn(sn, w);
+        }
+    }
+    return q;
+}
+
 // One CTA tile: voxels [tile * 128, tile * 128 + 128) of job `a`, all its transmits,
-// elements and frames.  `smem_words` is the dynamic shared memory (tx_chunk x 128 words,
+// elements and frames.  `smem_words` is the dynamic shared memory (tx_chunk x voxels words,
 // x3 in split mode).  Shared by the per-job kernel and the persistent batch kernel.
-// CS > 1 (one-frame jobs too small to fill the GPU): CS consecutive lanes share a voxel, each
-// summing every CS-th candidate element, and their sums are added with warp shuffles; a CTA
-// then covers 128 / CS voxels.
+// CS > 1 (one-frame jobs): CS lanes of a warp share a voxel, each summing every CS-th candidate
+// element, and their sums are added with warp shuffles; a CTA then covers 128 / CS voxels.  The
+// lanes of one element are consecutive (lane / (32 / CS) selects the element), so that the
+// lanes which a load serves together read one row, not CS rows.
 template <int S, int INTERP, int NF, bool SPLIT, int CS = 1>
 __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, float* smem_words, int chunk = 0) {
     static_assert(CS == 1 || NF == 1, "channel split: one-frame jobs only");
@@ -310,14 +477,17 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
     using T = typename ST::T;
     constexpr bool kCplx = ST::kComplex;
     constexpr unsigned kFull = 0xffffffffu;
-    // [tx_chunk][kLaneVoxelThreads] arrivals; split mode: sample base, fraction, phase cycles
+    constexpr int kVoxels = kLaneVoxelThreads / CS;  // voxels of the CTA
+    // [tx_chunk][kVoxels] arrivals; split mode: sample base, fraction, phase cycles
     float* const s_arrival = smem_words;
-    int* const s_base = reinterpret_cast<int*>(s_arrival + a.tx_chunk * kLaneVoxelThreads);
-    float* const s_cyc = s_arrival + 2 * a.tx_chunk * kLaneVoxelThreads;
+    int* const s_base = reinterpret_cast<int*>(s_arrival + a.tx_chunk * kVoxels);
+    float* const s_cyc = s_arrival + 2 * a.tx_chunk * kVoxels;
 
     const int lane = threadIdx.x & 31;
-    const int sub = threadIdx.x & (CS - 1);  // this lane's share of the voxel's elements
-    const int64_t v = lane_voxel_index<kLaneVoxelThreads / CS>(a, tile, threadIdx.x / CS);
+    constexpr int kLanesPerSub = 32 / CS;  // voxels of a warp
+    const int sub = lane / kLanesPerSub;   // this lane's share of the voxel's elements
+    const int lv = (threadIdx.x >> 5) * kLanesPerSub + (lane & (kLanesPerSub - 1));  // voxel of the tile
+    const int64_t v = lane_voxel_index<kVoxels>(a, tile, lv);
     const bool vox_ok = v < a.n_vox;
     const int n_frames = NF > 0 ? NF : a.n_frames;  // frames this thread sums
     // Frames per sample row, and this CTA's first frame: vector jobs with more frames than NF
@@ -364,11 +534,97 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
     const int row_len = a.n_samples * fstride;  // samples per (transmit, element) row
     const int tx_chunk = a.tx_chunk;
 
+    // Add the frames of one point: taps from tap 0 at p and (linear) the second tap at p1.
+    auto add_frames = [&](const T* p, const T* p1, const TapPosition& tp, float cw, float sw) {
+        if constexpr (kVec && !kCplx && INTERP != kQuadratic) {
+            // Real frames in pairs: the interpolation weights folded into the
+            // apodisation weight, acc += (1 - t) w a + t w b in packed FP32x2.
+            float2 va[kAcc];
+            load_frames<S, NF>(p, va);
+            if constexpr (INTERP == kLinear) {
+                float2 vb[kAcc];
+                load_frames<S, NF>(p1, vb);
+                const float wb = __fmul_rn(tp.w0, cw);
+                const float wa = __fsub_rn(cw, wb);
+#pragma unroll
+                for (int q = 0; q < kAcc; ++q) {
+                    acc[q] = __ffma2_rn(make_float2(wa, wa), va[q], acc[q]);
+                    acc[q] = __ffma2_rn(make_float2(wb, wb), vb[q], acc[q]);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < kAcc; ++q) acc[q] = __ffma2_rn(make_float2(cw, cw), va[q], acc[q]);
+            }
+            return;
+        }
+        if constexpr (kVec && kCplx && INTERP == kLinear && (S == kCF16 || S == kCBF16)) {
+            unsigned wa[NF], wb[NF];  // one (I, Q) word per frame
+            load_words<S, NF>(p, wa);
+            load_words<S, NF>(p1, wb);
+#pragma unroll
+            for (int q = 0; q < NF; ++q) {
+                const float2 x = lerp_half_word<S>(wa[q], wb[q], tp.w0);
+                acc[q].x = __fmaf_rn(x.x, cw, __fmaf_rn(-x.y, sw, acc[q].x));
+                acc[q].y = __fmaf_rn(x.y, cw, __fmaf_rn(x.x, sw, acc[q].y));
+            }
+            return;
+        }
+        if constexpr (kVec) {
+            float2 va[kAcc], vb[kAcc], vc[kAcc];
+            if constexpr (INTERP == kNearest) {
+                load_frames<S, NF>(p, va);
+            } else if constexpr (INTERP == kLinear) {
+                load_frames<S, NF>(p, va);
+                load_frames<S, NF>(p1, vb);
+            } else {
+                load_frames<S, NF>(p - fstride, va);
+                load_frames<S, NF>(p, vb);
+                load_frames<S, NF>(p + fstride, vc);
+            }
+#pragma unroll
+            for (int q = 0; q < kAcc; ++q) {
+                float2 x;
+                if constexpr (INTERP == kNearest) {
+                    x = va[q];
+                } else if constexpr (INTERP == kLinear) {
+                    x.x = __fmaf_rn(tp.w0, __fsub_rn(vb[q].x, va[q].x), va[q].x);
+                    x.y = __fmaf_rn(tp.w0, __fsub_rn(vb[q].y, va[q].y), va[q].y);
+                } else {
+                    x.x = __fmaf_rn(tp.w2, vc[q].x, __fmaf_rn(tp.w0, va[q].x, __fmul_rn(tp.w1, vb[q].x)));
+                    x.y = __fmaf_rn(tp.w2, vc[q].y, __fmaf_rn(tp.w0, va[q].y, __fmul_rn(tp.w1, vb[q].y)));
+                }
+                if constexpr (kCplx) {
+                    acc[q].x = __fmaf_rn(x.x, cw, __fmaf_rn(-x.y, sw, acc[q].x));
+                    acc[q].y = __fmaf_rn(x.y, cw, __fmaf_rn(x.x, sw, acc[q].y));
+                } else {
+                    acc[q].x = __fmaf_rn(x.x, cw, acc[q].x);
+                    acc[q].y = __fmaf_rn(x.y, cw, acc[q].y);
+                }
+            }
+            return;
+        }
+#pragma unroll
+        for (int f = 0; f < kAcc; ++f) {
+            if (NF > 0 || f < n_frames) {
+                const float2 x = tap_value<S, INTERP>(p + f, p1 + f, tp, n_frames);
+                if constexpr (kCplx) {
+                    acc[f].x = __fmaf_rn(x.x, cw, __fmaf_rn(-x.y, sw, acc[f].x));
+                    acc[f].y = __fmaf_rn(x.y, cw, __fmaf_rn(x.x, sw, acc[f].y));
+                } else {
+                    acc[f].x = __fmaf_rn(x.x, cw, acc[f].x);
+                }
+            }
+        }
+    };
+
     for (int t0 = 0; t0 < a.n_tx; t0 += tx_chunk) {
         const int nt = min(tx_chunk, a.n_tx - t0);
+        TxRange<SPLIT> tx_range;
         __syncthreads();
-        for (int i = threadIdx.x; i < nt * kLaneVoxelThreads; i += kLaneVoxelThreads) {
-            const int t = i / kLaneVoxelThreads;  // i - t * 128 is this thread's index: its own voxel
+        // Each voxel's lanes stage its arrivals (every CS-th transmit each); the copy is shared, and
+        // the range is combined over the lanes.
+        for (int t = sub; t < nt; t += CS) {
+            const int i = t * kVoxels + lv;
             const float txa = vox_ok ? __ldg(a.arrivals + static_cast<int64_t>(t0 + t) * a.n_vox + v) : 0.f;
             if constexpr (SPLIT) {
                 // transmit part of the sample position and phase, per (voxel, transmit)
@@ -376,10 +632,14 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
                 s_base[i] = sp.base;
                 s_arrival[i] = sp.frac;
                 s_cyc[i] = reduced_cycles(static_cast<double>(txa) * a.fmod_d);
+                tx_range.add(txa, sp.base);
             } else {
                 s_arrival[i] = txa;
+                tx_range.add(txa, 0);
             }
         }
+#pragma unroll
+        for (int off = kLanesPerSub; off < 32; off <<= 1) tx_range.merge(off);
         __syncthreads();
 
         for (int eb = a.e_begin; eb < a.e_end; eb += 32) {
@@ -429,6 +689,66 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
 
                 int row = (t0 * a.n_rx + e) * row_len;
                 const int tx_step = a.n_rx * row_len;
+                // Every point of every lane inside its row: the transmit loop without tests.  The loop is
+                // bound by instruction issue, and the range tests, their selects and the row index
+                // were a third to a half of a one-frame point's instructions.  Measured on B200, same
+                // bits: one 128^3 volume of int16 from 1024 elements and 9 transmits (split delays)
+                // 32.0 -> 21.5 ms, 16 frames of it 68.5 -> 61.7 ms, 11 transmits of FP16 pairs on
+                // 301 x 397 0.28 -> 0.23 ms, 75 transmits of complex64 1.71 -> 1.51 ms (with the lane
+                // order above, which took its L1 data pipe from 96 % to 56 %).
+                if (__all_sync(kFull, !pair_ok || taps_always_inside<INTERP, SPLIT>(a, tx_range, dist, rx_pos))) {
+                    if (pair_ok) {
+                        const unsigned sample_bytes = static_cast<unsigned>(fstride * static_cast<int>(sizeof(T)));
+                        const char* rp = safe_row<SPLIT>(channel + (static_cast<int64_t>(row) + f0), sample_bytes);
+                        const int64_t rp_step = static_cast<int64_t>(tx_step) * static_cast<int64_t>(sizeof(T));
+                        const float* sa = s_arrival + lv;
+                        const int* sb = s_base + lv;
+                        const float* sc = s_cyc + lv;
+                        auto point_at = [&](int t, const char* r) {
+                            const int si = t * kVoxels;
+                            return safe_point<INTERP, SPLIT, kCplx, S == kI16 || S == kCI16>(
+                                a, r, NF == 1 ? static_cast<unsigned>(sizeof(T)) : sample_bytes, dist, rx_pos, rx_cyc,
+                                w, sa[si], SPLIT ? sb[si] : 0, SPLIT ? sc[si] : 0.f);
+                        };
+                        if constexpr (NF == 1) {
+                            auto add_one = [&](const SafePoint& q, float2 x) {
+                                if constexpr (kDeferRot) {
+                                    acc_c = __ffma2_rn(make_float2(q.cw, q.cw), x, acc_c);
+                                    acc_s = __ffma2_rn(make_float2(q.sw, q.sw), x, acc_s);
+                                } else if constexpr (kCplx) {
+                                    acc[0].x = __fmaf_rn(x.x, q.cw, __fmaf_rn(-x.y, q.sw, acc[0].x));
+                                    acc[0].y = __fmaf_rn(x.y, q.cw, __fmaf_rn(x.x, q.sw, acc[0].y));
+                                } else {
+                                    acc[0].x = __fmaf_rn(x.x, q.cw, acc[0].x);
+                                }
+                            };
+                            auto value = [&](const SafePoint& q) {
+                                return tap_value<S, INTERP, kDeferRot>(reinterpret_cast<const T*>(q.p0),
+                                                                       reinterpret_cast<const T*>(q.p1), q.tp, 1);
+                            };
+                            int t = 0;
+#pragma unroll 1
+                            for (; t + 1 < nt; t += 2, rp += 2 * rp_step) {  // both transmits' loads in flight
+                                const SafePoint qa = point_at(t, rp), qb = point_at(t + 1, rp + rp_step);
+                                const float2 xa = value(qa), xb = value(qb);
+                                add_one(qa, xa);
+                                add_one(qb, xb);
+                            }
+                            if (t < nt) {
+                                const SafePoint qa = point_at(t, rp);
+                                add_one(qa, value(qa));
+                            }
+                        } else {
+#pragma unroll 1
+                            for (int t = 0; t < nt; ++t, rp += rp_step) {
+                                const SafePoint q = point_at(t, rp);
+                                add_frames(reinterpret_cast<const T*>(q.p0), reinterpret_cast<const T*>(q.p1), q.tp,
+                                           q.cw, q.sw);
+                            }
+                        }
+                    }
+                    continue;
+                }
                 if constexpr (NF == 1) {
                     if (a.n_samples >= 3) {
                         // Two transmits at a time with no branch between them, so that the
@@ -442,7 +762,7 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
 #pragma unroll
                             for (int u = 0; u < 2; ++u) {
                                 const bool in = t + u < nt;
-                                const int si = (in ? t + u : t) * kLaneVoxelThreads + threadIdx.x;
+                                const int si = (in ? t + u : t) * kVoxels + lv;
                                 TapPosition tp{};
                                 bool ok;
                                 float cw = w, sw = 0.f;
@@ -488,7 +808,8 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
                                     tp.step = 0;
                                 }
                                 const int row_u = in ? row + u * tx_step : row;
-                                xv[u] = tap_value<S, INTERP, kDeferRot>(channel + (row_u + tp.idx * n_frames), tp, n_frames);
+                                const T* pt = channel + (row_u + tp.idx);
+                                xv[u] = tap_value<S, INTERP, kDeferRot>(pt, pt + tp.step, tp, 1);
                                 cwv[u] = cw;
                                 swv[u] = sw;
                                 okv[u] = ok;
@@ -518,7 +839,7 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
                 }
 #pragma unroll 2
                 for (int t = 0; t < nt; ++t, row += tx_step) {
-                    const int si = t * kLaneVoxelThreads + threadIdx.x;
+                    const int si = t * kVoxels + lv;
                     TapPosition tp;
                     float cw = w, sw = 0.f;
                     if constexpr (SPLIT) {
@@ -563,85 +884,7 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
                         }
                     }
                     const T* p = channel + (row + tp.idx * fstride + f0);
-                    if constexpr (kVec && !kCplx && INTERP != kQuadratic) {
-                        // Real frames in pairs: the interpolation weights folded into the
-                        // apodisation weight, acc += (1 - t) w a + t w b in packed FP32x2.
-                        float2 va[kAcc];
-                        load_frames<S, NF>(p, va);
-                        if constexpr (INTERP == kLinear) {
-                            float2 vb[kAcc];
-                            load_frames<S, NF>(p + tp.step * fstride, vb);
-                            const float wb = __fmul_rn(tp.w0, cw);
-                            const float wa = __fsub_rn(cw, wb);
-#pragma unroll
-                            for (int q = 0; q < kAcc; ++q) {
-                                acc[q] = __ffma2_rn(make_float2(wa, wa), va[q], acc[q]);
-                                acc[q] = __ffma2_rn(make_float2(wb, wb), vb[q], acc[q]);
-                            }
-                        } else {
-#pragma unroll
-                            for (int q = 0; q < kAcc; ++q) acc[q] = __ffma2_rn(make_float2(cw, cw), va[q], acc[q]);
-                        }
-                        continue;
-                    }
-                    if constexpr (kVec && kCplx && INTERP == kLinear && (S == kCF16 || S == kCBF16)) {
-                        unsigned wa[NF], wb[NF];  // one (I, Q) word per frame
-                        load_words<S, NF>(p, wa);
-                        load_words<S, NF>(p + tp.step * fstride, wb);
-#pragma unroll
-                        for (int q = 0; q < NF; ++q) {
-                            const float2 x = lerp_half_word<S>(wa[q], wb[q], tp.w0);
-                            acc[q].x = __fmaf_rn(x.x, cw, __fmaf_rn(-x.y, sw, acc[q].x));
-                            acc[q].y = __fmaf_rn(x.y, cw, __fmaf_rn(x.x, sw, acc[q].y));
-                        }
-                        continue;
-                    }
-                    if constexpr (kVec) {
-                        float2 va[kAcc], vb[kAcc], vc[kAcc];
-                        if constexpr (INTERP == kNearest) {
-                            load_frames<S, NF>(p, va);
-                        } else if constexpr (INTERP == kLinear) {
-                            load_frames<S, NF>(p, va);
-                            load_frames<S, NF>(p + tp.step * fstride, vb);
-                        } else {
-                            load_frames<S, NF>(p - fstride, va);
-                            load_frames<S, NF>(p, vb);
-                            load_frames<S, NF>(p + fstride, vc);
-                        }
-#pragma unroll
-                        for (int q = 0; q < kAcc; ++q) {
-                            float2 x;
-                            if constexpr (INTERP == kNearest) {
-                                x = va[q];
-                            } else if constexpr (INTERP == kLinear) {
-                                x.x = __fmaf_rn(tp.w0, __fsub_rn(vb[q].x, va[q].x), va[q].x);
-                                x.y = __fmaf_rn(tp.w0, __fsub_rn(vb[q].y, va[q].y), va[q].y);
-                            } else {
-                                x.x = __fmaf_rn(tp.w2, vc[q].x, __fmaf_rn(tp.w0, va[q].x, __fmul_rn(tp.w1, vb[q].x)));
-                                x.y = __fmaf_rn(tp.w2, vc[q].y, __fmaf_rn(tp.w0, va[q].y, __fmul_rn(tp.w1, vb[q].y)));
-                            }
-                            if constexpr (kCplx) {
-                                acc[q].x = __fmaf_rn(x.x, cw, __fmaf_rn(-x.y, sw, acc[q].x));
-                                acc[q].y = __fmaf_rn(x.y, cw, __fmaf_rn(x.x, sw, acc[q].y));
-                            } else {
-                                acc[q].x = __fmaf_rn(x.x, cw, acc[q].x);
-                                acc[q].y = __fmaf_rn(x.y, cw, acc[q].y);
-                            }
-                        }
-                        continue;
-                    }
-#pragma unroll
-                    for (int f = 0; f < kAcc; ++f) {
-                        if (NF > 0 || f < n_frames) {
-                            const float2 x = tap_value<S, INTERP>(p + f, tp, n_frames);
-                            if constexpr (kCplx) {
-                                acc[f].x = __fmaf_rn(x.x, cw, __fmaf_rn(-x.y, sw, acc[f].x));
-                                acc[f].y = __fmaf_rn(x.y, cw, __fmaf_rn(x.x, sw, acc[f].y));
-                            } else {
-                                acc[f].x = __fmaf_rn(x.x, cw, acc[f].x);
-                            }
-                        }
-                    }
+                    add_frames(p, p + tp.step * fstride, tp, cw, sw);
                 }
             }
         }
@@ -653,7 +896,7 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
     }
     if constexpr (CS > 1) {  // add the lanes' partial sums of each voxel
 #pragma unroll
-        for (int off = 1; off < CS; off <<= 1) {
+        for (int off = kLanesPerSub; off < 32; off <<= 1) {
 #pragma unroll
             for (int f = 0; f < kAcc; ++f) {
                 acc[f].x = __fadd_rn(acc[f].x, __shfl_xor_sync(kFull, acc[f].x, off));
@@ -808,8 +1051,18 @@ __device__ __forceinline__ float2 gather_taps(const typename Storage<S>::T* row,
     }
 }
 
+// CTAs per SM that the register budget is cut for, from the state a point keeps live: 16 frames of
+// 16-bit real samples fit 72 registers, of float32 96, of complex samples 128; 8 complex64 frames 72
+// (quadratic: three rows in flight, 96); the other kernels 64.
+template <int S, int INTERP, int NF>
+constexpr int lane_voxel_ctas() {
+    if (NF == 16) return Storage<S>::kComplex ? 4 : (S == kF32 ? 5 : 7);
+    if (NF == 8 && S == kC64) return INTERP == kQuadratic ? 5 : 7;
+    return 8;
+}
+
 template <int S, int INTERP, int NF, bool SPLIT, int CS = 1>
-__global__ void __launch_bounds__(kLaneVoxelThreads, NF == 16 ? 4 : 8)
+__global__ void __launch_bounds__(kLaneVoxelThreads, lane_voxel_ctas<S, INTERP, NF>())
     das_lane_voxel_kernel(const __grid_constant__ DasArgs a) {
     extern __shared__ float smem_words[];
     if (NF >= 2 && a.frame_chunks > 1) {  // consecutive CTAs: the chunks of one tile, which share rows

@@ -196,10 +196,12 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 
 // ---------------------------------------------------------------- launch planning
 
-// Lane-voxel kernel: transmits whose arrivals a CTA stages at once (40 x 128 voxels x 4 B = 20 KB,
-// nine CTAs per SM; split delays stage three words per entry, so 32).  A job of n_tx transmits
-// runs in ceil(n_tx / cap) equal passes over its elements (75 transmits: 2 passes of 38 and 37;
-// measured on B200, compounding 1.64 ms against 1.71 ms with 3 passes of 25).
+// Lane-voxel kernel: transmits whose arrivals a CTA of 128 voxels stages at once (40 x 128 voxels x
+// 4 B = 20 KB, nine CTAs per SM; split delays stage three words per entry, so 32).  With 2 or 4
+// lanes per voxel a CTA has 64 or 32 voxels and stages 2 or 4 times as many transmits in the same
+// memory.  A job of n_tx transmits runs in ceil(n_tx / cap) equal passes over its elements: the
+// receive path of a (voxel, element) pair is computed once per pass (measured on B200, 75
+// transmits of compounding with 2 lanes: one pass 1.44 ms, two 1.50 ms, three 1.56 ms).
 constexpr int kMaxTxChunk = 40;
 constexpr int kMaxTxChunkSplit = 32;
 
@@ -422,10 +424,6 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
         p.lp.kind = n_frames <= 1 ? kKindLaneVoxel1 : (n_frames == 16 ? kKindLaneVoxel16 : kKindLaneVoxelN);
         if (n_frames > 16) p.lp.kind = kKindLaneVoxel8;  // lane8_ok (checked above)
         p.lp.passes = static_cast<int>(n_frames);
-        const int chunk = o.tx_chunk > 0 ? o.tx_chunk
-                                         : ((o.flags & MACH_B200_FLAG_SPLIT_DELAY) ? kMaxTxChunkSplit : kMaxTxChunk);
-        const uint32_t chunks = std::max<uint32_t>(1u, (n_tx + chunk - 1) / chunk);
-        p.lp.tx_chunk = static_cast<int>(std::max<uint32_t>(1u, (n_tx + chunks - 1) / chunks));
         p.lp.block = dim3(kLaneVoxelThreads, 1, 1);
         // One-frame jobs split each voxel's elements over 2 or 4 lanes.  Measured on B200: 4
         // for jobs of fewer than 4 CTAs of 128 voxels per SM and for split delays, 2 otherwise.
@@ -440,6 +438,10 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
         }
         p.lp.lanes_per_voxel = cs;
         const int vpc = kLaneVoxelThreads / cs;  // voxels per CTA
+        const int chunk = o.tx_chunk > 0 ? o.tx_chunk
+                                         : cs * ((o.flags & MACH_B200_FLAG_SPLIT_DELAY) ? kMaxTxChunkSplit : kMaxTxChunk);
+        const uint32_t chunks = std::max<uint32_t>(1u, (n_tx + chunk - 1) / chunk);
+        p.lp.tx_chunk = static_cast<int>(std::max<uint32_t>(1u, (n_tx + chunks - 1) / chunks));
         p.lp.grid = dim3(static_cast<unsigned>((n_vox + vpc - 1) / vpc), 1, 1);
         // On a known grid: CTA tiles of wf x (128 / wf) voxels, warps of wf x (32 / wf).
         // Automatic: 2 along the contiguous axis for 16 frames (rows of 32+ bytes), else 4.
@@ -478,7 +480,7 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
             p.lp.element_block = eb > 0 ? eb : 0;
         }
         // split mode stages three words per (transmit, voxel): base, fraction, phase cycles
-        p.lp.smem = static_cast<size_t>(p.lp.tx_chunk) * kLaneVoxelThreads * sizeof(float) *
+        p.lp.smem = static_cast<size_t>(p.lp.tx_chunk) * vpc * sizeof(float) *
                     ((o.flags & MACH_B200_FLAG_SPLIT_DELAY) ? 3 : 1);
         return p;
     }
