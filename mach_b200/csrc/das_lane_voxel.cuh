@@ -193,13 +193,29 @@ __device__ __forceinline__ void widen8<kI16>(uint2 r, float2* o) {
     widen8<kCI16>(r, o);
 }
 
-// Load the NF frames of one sample (NF * sizeof(T) is a multiple of 16 bytes).  Rows of a
-// multiple of 32 bytes are read with 256-bit loads, so that each lane's request covers whole
-// 32-byte sectors (the planner only runs them on 32-byte aligned rows; measured on B200:
-// Doppler complex64 in 8-frame chunks 5.7 -> 4.0 ms, FP16 3.45 -> 3.30 ms); others with
+// 32-byte pieces of the NF frames of one sample; a lane starts with piece `first` and takes the
+// others in turn (piece i of a lane is (i ^ first)).
+template <int S, int NF>
+struct FramePieces {
+    static constexpr int kBytes = NF * static_cast<int>(sizeof(typename Storage<S>::T));
+    static constexpr int kCount = kBytes % 32 == 0 ? kBytes / 32 : 1;
+    // The first piece of this lane.  The 32 bytes that each of four neighbouring lanes reads lie in
+    // different sample rows, often at the same offset of a 128-byte line; starting some lanes with
+    // another piece spreads the four over the line's banks.
+    __device__ static __forceinline__ int first(int lane) {
+        if constexpr (kCount == 2) return (lane >> 1) & 1;
+        if constexpr (kCount == 4) return lane & 3;
+        return 0;
+    }
+};
+
+// Load the NF frames of one sample (NF * sizeof(T) is a multiple of 16 bytes), piece by piece from
+// `first`.  Rows of a multiple of 32 bytes are read with 256-bit loads, so that each lane's request
+// covers whole 32-byte sectors (the planner only runs them on 32-byte aligned rows; measured on
+// B200: Doppler complex64 in 8-frame chunks 5.7 -> 4.0 ms, FP16 3.45 -> 3.30 ms); others with
 // 128-bit loads.
 template <int S, int NF>
-__device__ __forceinline__ void load_frames(const typename Storage<S>::T* p, float2* o) {
+__device__ __forceinline__ void load_frames(const typename Storage<S>::T* p, float2* o, int first) {
     constexpr int kBytes = NF * static_cast<int>(sizeof(typename Storage<S>::T));
     static_assert(kBytes % 16 == 0, "vector frames need 16-byte rows");
     constexpr int kPairsPer8 = FramePairs<S, NF>::kValue / (kBytes / 8);
@@ -209,7 +225,7 @@ __device__ __forceinline__ void load_frames(const typename Storage<S>::T* p, flo
             unsigned r[8];
             asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                : "l"(reinterpret_cast<const char*>(p) + 32 * i));
+                : "l"(reinterpret_cast<const char*>(p) + 32 * (kBytes == 32 ? i : (i ^ first))));
 #pragma unroll
             for (int k = 0; k < 4; ++k) widen8<S>(make_uint2(r[2 * k], r[2 * k + 1]), o + (4 * i + k) * kPairsPer8);
         }
@@ -227,7 +243,7 @@ __device__ __forceinline__ void load_frames(const typename Storage<S>::T* p, flo
 // Raw 32-bit words of the NF frames of one sample (NF * sizeof(T) bytes, a multiple of 16;
 // 256-bit loads when a multiple of 32, as load_frames).
 template <int S, int NF>
-__device__ __forceinline__ void load_words(const typename Storage<S>::T* p, unsigned* w) {
+__device__ __forceinline__ void load_words(const typename Storage<S>::T* p, unsigned* w, int first) {
     constexpr int kBytes = NF * static_cast<int>(sizeof(typename Storage<S>::T));
     static_assert(kBytes % 16 == 0, "vector frames need 16-byte rows");
     if constexpr (kBytes % 32 == 0) {
@@ -236,7 +252,7 @@ __device__ __forceinline__ void load_words(const typename Storage<S>::T* p, unsi
             unsigned* r = w + 8 * i;
             asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-                : "l"(reinterpret_cast<const char*>(p) + 32 * i));
+                : "l"(reinterpret_cast<const char*>(p) + 32 * (kBytes == 32 ? i : (i ^ first))));
         }
     } else {
         const uint4* q = reinterpret_cast<const uint4*>(p);
@@ -534,16 +550,18 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
     const int row_len = a.n_samples * fstride;  // samples per (transmit, element) row
     const int tx_chunk = a.tx_chunk;
 
+    const int first_piece = kVec ? FramePieces<S, NF>::first(lane) : 0;
+
     // Add the frames of one point: taps from tap 0 at p and (linear) the second tap at p1.
     auto add_frames = [&](const T* p, const T* p1, const TapPosition& tp, float cw, float sw) {
         if constexpr (kVec && !kCplx && INTERP != kQuadratic) {
             // Real frames in pairs: the interpolation weights folded into the
             // apodisation weight, acc += (1 - t) w a + t w b in packed FP32x2.
             float2 va[kAcc];
-            load_frames<S, NF>(p, va);
+            load_frames<S, NF>(p, va, first_piece);
             if constexpr (INTERP == kLinear) {
                 float2 vb[kAcc];
-                load_frames<S, NF>(p1, vb);
+                load_frames<S, NF>(p1, vb, first_piece);
                 const float wb = __fmul_rn(tp.w0, cw);
                 const float wa = __fsub_rn(cw, wb);
 #pragma unroll
@@ -559,8 +577,8 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
         }
         if constexpr (kVec && kCplx && INTERP == kLinear && (S == kCF16 || S == kCBF16)) {
             unsigned wa[NF], wb[NF];  // one (I, Q) word per frame
-            load_words<S, NF>(p, wa);
-            load_words<S, NF>(p1, wb);
+            load_words<S, NF>(p, wa, first_piece);
+            load_words<S, NF>(p1, wb, first_piece);
 #pragma unroll
             for (int q = 0; q < NF; ++q) {
                 const float2 x = lerp_half_word<S>(wa[q], wb[q], tp.w0);
@@ -572,14 +590,14 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
         if constexpr (kVec) {
             float2 va[kAcc], vb[kAcc], vc[kAcc];
             if constexpr (INTERP == kNearest) {
-                load_frames<S, NF>(p, va);
+                load_frames<S, NF>(p, va, first_piece);
             } else if constexpr (INTERP == kLinear) {
-                load_frames<S, NF>(p, va);
-                load_frames<S, NF>(p1, vb);
+                load_frames<S, NF>(p, va, first_piece);
+                load_frames<S, NF>(p1, vb, first_piece);
             } else {
-                load_frames<S, NF>(p - fstride, va);
-                load_frames<S, NF>(p, vb);
-                load_frames<S, NF>(p + fstride, vc);
+                load_frames<S, NF>(p - fstride, va, first_piece);
+                load_frames<S, NF>(p, vb, first_piece);
+                load_frames<S, NF>(p + fstride, vc, first_piece);
             }
 #pragma unroll
             for (int q = 0; q < kAcc; ++q) {
@@ -907,10 +925,12 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
     }
     if (!vox_ok) return;
     if constexpr (kVec) {
+        constexpr int kPerPiece = kAcc / FramePieces<S, NF>::kCount;  // sums of one piece
 #pragma unroll
         for (int q = 0; q < kAcc; ++q) {
+            const int at = ((q / kPerPiece) ^ first_piece) * kPerPiece + q % kPerPiece;  // its place in the row
             if constexpr (kCplx) {
-                float2* out = static_cast<float2*>(a.out) + v * fstride + f0 + q;
+                float2* out = static_cast<float2*>(a.out) + v * fstride + f0 + at;
                 float2 r = acc[q];
                 if (a.accumulate) {
                     const float2 prev = *out;
@@ -919,7 +939,7 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
                 }
                 *out = r;
             } else {
-                float* out = static_cast<float*>(a.out) + v * fstride + f0 + 2 * q;
+                float* out = static_cast<float*>(a.out) + v * fstride + f0 + 2 * at;
                 out[0] = a.accumulate ? __fadd_rn(out[0], acc[q].x) : acc[q].x;
                 out[1] = a.accumulate ? __fadd_rn(out[1], acc[q].y) : acc[q].y;
             }
