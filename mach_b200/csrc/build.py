@@ -48,7 +48,7 @@ def _flags() -> list[str]:
 
 
 def _headers() -> list[Path]:
-    return sorted(CSRC.glob("*.cuh")) + [REPO / "include" / "mach_b200.h"]
+    return sorted(CSRC.glob("*.cuh")) + sorted(CSRC.glob("*.h")) + [REPO / "include" / "mach_b200.h"]
 
 
 def _compile(src: Path, flags: list[str], force: bool) -> tuple[Path, str]:

@@ -140,7 +140,11 @@ struct DasArgs {
     // deepest first for a depth-fastest scan, whose wide apertures make them the heaviest), so the
     // CTAs that start last take light tiles; 0: grid order (outer-major).
     int32_t tile_rev;
-    int32_t frame_chunks;   // lane-voxel 8-frame chunks: CTA b takes tile b / frame_chunks, chunk b % frame_chunks
+    int32_t frame_chunks;   // lane-voxel chunks of 8 or 16 frames: CTA b takes tile b / frame_chunks, chunk b % frame_chunks
+    int32_t row_frames;     // lane-voxel kernels: frames stored per sample (n_frames; more in a padded copy)
+    // Lane-voxel kernels without a known grid: device word with the contiguous extent that
+    // das_probe_grid_kernel found (0: none), read instead of map_fast; nullptr otherwise.
+    const int32_t* probed_fast;
     int32_t e_begin;        // lane-voxel kernels: elements [e_begin, e_end) of this launch
     int32_t e_end;
     int32_t start_base;     // floor(-t0 * fs): samples before it belong to tau < 0

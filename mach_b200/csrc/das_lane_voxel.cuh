@@ -201,7 +201,8 @@ struct FramePieces {
     static constexpr int kCount = kBytes % 32 == 0 ? kBytes / 32 : 1;
     // The first piece of this lane.  The 32 bytes that each of four neighbouring lanes reads lie in
     // different sample rows, often at the same offset of a 128-byte line; starting some lanes with
-    // another piece spreads the four over the line's banks.
+    // another piece spreads the four over the line's banks (200-frame complex64 Doppler on B200:
+    // L1 data pipe 94 -> 72 % busy, 3.77 -> 3.67 ms; load latency bounds it now).
     __device__ static __forceinline__ int first(int lane) {
         if constexpr (kCount == 2) return (lane >> 1) & 1;
         if constexpr (kCount == 4) return lane & 3;
@@ -308,14 +309,21 @@ __device__ __forceinline__ float fast_tukey(float h2, float radius, const DasArg
 // together in memory (few L1 lines per warp load); otherwise a tile is 128 consecutive voxels.
 template <int VPC = kLaneVoxelThreads>
 __device__ __forceinline__ int64_t lane_voxel_index(const DasArgs& a, int64_t tile, int j) {
-    if (a.map_fast <= 0) return tile * VPC + j;
+    int map_fast = a.map_fast;
+    int64_t map_outer = a.map_outer;
+    if (a.probed_fast != nullptr) {  // contiguous extent found on the device (das_probe_grid_kernel)
+        map_fast = *a.probed_fast;
+        map_outer = map_fast > 0 ? a.n_vox / map_fast : 0;
+    }
+    if (map_fast <= 0) return tile * VPC + j;
     const int lw = a.map_wlog;
-    const int64_t tiles_fast = (a.map_fast + (1 << lw) - 1) >> lw;
+    const int64_t tiles_fast = (map_fast + (1 << lw) - 1) >> lw;
     const int64_t per_outer = VPC >> lw;  // outer-axis voxels of a tile
     int64_t to, tf;                        // the tile's outer and fast-axis tile coordinates
     if (a.tile_rev) {
-        const int64_t tiles_outer = (a.map_outer + per_outer - 1) / per_outer;
+        const int64_t tiles_outer = (map_outer + per_outer - 1) / per_outer;
         const int64_t q = tile / tiles_outer;
+        if (q >= tiles_fast) return a.n_vox;  // launched for a bound of the tiles (probed grids)
         to = tile - q * tiles_outer;
         tf = tiles_fast - 1 - q;
     } else {
@@ -324,7 +332,7 @@ __device__ __forceinline__ int64_t lane_voxel_index(const DasArgs& a, int64_t ti
     }
     const int64_t o = to * per_outer + (j >> lw);
     const int64_t f = (tf << lw) + (j & ((1 << lw) - 1));
-    return (o < a.map_outer && f < a.map_fast) ? o * a.map_fast + f : a.n_vox;
+    return (o < map_outer && f < map_fast) ? o * map_fast + f : a.n_vox;
 }
 
 // min / max that return NaN when either operand is one (a NaN arrival must fail the range test).
@@ -505,10 +513,11 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
     const int lv = (threadIdx.x >> 5) * kLanesPerSub + (lane & (kLanesPerSub - 1));  // voxel of the tile
     const int64_t v = lane_voxel_index<kVoxels>(a, tile, lv);
     const bool vox_ok = v < a.n_vox;
+    if (NF >= 2 && a.probed_fast != nullptr && !__syncthreads_or(vox_ok)) return;
     const int n_frames = NF > 0 ? NF : a.n_frames;  // frames this thread sums
-    // Frames per sample row, and this CTA's first frame: vector jobs with more frames than NF
-    // run in chunks of NF frames.
-    const int fstride = a.n_frames;
+    // Frames stored per sample row (n_frames, or more in a padded copy), and this CTA's first frame:
+    // vector jobs with more frames than NF run in chunks of NF frames.
+    const int fstride = a.row_frames;
     const int f0 = NF >= 2 ? chunk * NF : 0;
 
     float vx = 0.f, vy = 0.f, vz = 0.f;
@@ -930,7 +939,8 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
         for (int q = 0; q < kAcc; ++q) {
             const int at = ((q / kPerPiece) ^ first_piece) * kPerPiece + q % kPerPiece;  // its place in the row
             if constexpr (kCplx) {
-                float2* out = static_cast<float2*>(a.out) + v * fstride + f0 + at;
+                if (f0 + at >= a.n_frames) continue;  // padding of the last chunk
+                float2* out = static_cast<float2*>(a.out) + v * a.n_frames + f0 + at;
                 float2 r = acc[q];
                 if (a.accumulate) {
                     const float2 prev = *out;
@@ -939,9 +949,10 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
                 }
                 *out = r;
             } else {
-                float* out = static_cast<float*>(a.out) + v * fstride + f0 + 2 * at;
-                out[0] = a.accumulate ? __fadd_rn(out[0], acc[q].x) : acc[q].x;
-                out[1] = a.accumulate ? __fadd_rn(out[1], acc[q].y) : acc[q].y;
+                const int f = f0 + 2 * at;
+                float* out = static_cast<float*>(a.out) + v * a.n_frames + f;
+                if (f < a.n_frames) out[0] = a.accumulate ? __fadd_rn(out[0], acc[q].x) : acc[q].x;
+                if (f + 1 < a.n_frames) out[1] = a.accumulate ? __fadd_rn(out[1], acc[q].y) : acc[q].y;
             }
         }
         return;

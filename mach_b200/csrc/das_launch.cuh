@@ -12,13 +12,20 @@
 
 namespace mach_b200 {
 
+// Instances of the 16-frame lane-voxel kernels: the plans that ask for them (plan_launch) are real
+// storage and complex64 with one or two taps.
+template <int S, int I>
+constexpr bool lane_voxel_has16() {
+    return !Storage<S>::kComplex || (S == kC64 && I != kQuadratic);
+}
+
 enum KernelKind : int {
     kKindLaneVoxel1 = 0,   // das_lane_voxel_kernel, exactly one frame
     kKindLaneVoxelN = 1,   // das_lane_voxel_kernel, 2..8 frames per lane
     kKindWarpHalf = 2,     // das_gather_kernel, 16 lanes per voxel
     kKindWarp = 3,         // das_gather_kernel, 32 lanes per voxel
     kKindStaged = 4,       // das_staged_kernel, windows staged in shared memory (TMA or direct)
-    kKindLaneVoxel16 = 5,  // das_lane_voxel_kernel, exactly 16 frames loaded as 16-byte vectors
+    kKindLaneVoxel16 = 5,  // das_lane_voxel_kernel, 16 frames (or chunks of 16) loaded as vectors
     kKindEnsemble = 6,     // das_ensemble_kernel, windows in tensor memory, lanes = frames
     kKindLaneVoxel8 = 7,   // das_lane_voxel_kernel, chunks of 8 frames (grid.y) of a longer ensemble
     kKindFrameLane = 8,    // das_frame_lane_kernel, lanes = frames, rows reused along voxel runs
@@ -36,7 +43,9 @@ struct LaunchPlan {
     int map_wlog;
     int64_t map_outer;
     int tile_rev;       // lane-voxel kernels on a grid: far end of the contiguous axis first (DasArgs::tile_rev)
-    int frame_chunks;   // lane-voxel 8-frame chunks per tile (DasArgs::frame_chunks)
+    int frame_chunks;   // lane-voxel chunks of 8 or 16 frames per tile (DasArgs::frame_chunks)
+    int pad_frames;     // lane-voxel kernels: frames per sample of the padded copy to run on, 0 = none
+    bool probe_grid;    // lane-voxel kernels: tile by the extent that a probe of the scan points finds
     int element_block;  // lane-voxel kernels: elements per launch (0 = all), so that one launch's
                         // channel data stays resident in L2
     int frame_slots;    // frame-lane kernel: J, lane-word columns per warp (1, 2 or 4)
@@ -109,7 +118,9 @@ cudaError_t launch_das(const DasArgs& a, int interp, const LaunchPlan& p, cudaSt
             else MACH_B200_LV(I, 1);                         \
             break;                                           \
         case kKindLaneVoxelN: MACH_B200_LV(I, 0); break;     \
-        case kKindLaneVoxel16: MACH_B200_LV(I, 16); break;   \
+        case kKindLaneVoxel16:                               \
+            if constexpr (lane_voxel_has16<S, I>()) MACH_B200_LV(I, 16); \
+            break;                                           \
         case kKindLaneVoxel8: MACH_B200_LV(I, 8); break;     \
         case kKindWarpHalf: MACH_B200_WG(I, 16, 4); break;   \
         default: MACH_B200_WG(I, 32, 8); break;              \
@@ -190,7 +201,9 @@ cudaError_t launch_lane_voxel_persistent(int interp, int frame_class, bool split
         case 1: MACH_B200_PLV(I, 1, 1);             \
         case 12: MACH_B200_PLV(I, 1, 2);            \
         case 14: MACH_B200_PLV(I, 1, 4);            \
-        case 16: MACH_B200_PLV(I, 16, 1);           \
+        case 16:                                    \
+            if constexpr (lane_voxel_has16<S, I>()) {MACH_B200_PLV(I, 16, 1);} \
+            return cudaErrorInvalidValue;           \
         case 8: MACH_B200_PLV(I, 8, 1);             \
         default: MACH_B200_PLV(I, 0, 1);            \
     }
@@ -290,6 +303,15 @@ cudaError_t launch_hilbert(int src_code, int dst_code, const HilbertArgs& g, siz
 // device memory.
 cudaError_t launch_tx_arrivals(int model, const double* params, const float* scan, int64_t n_scan, int n_tx,
                                double sound_speed, float* out, cudaStream_t st);
+
+// Layout helpers of the lane-voxel kernels (das_layout.cu).
+// Copy rows of n frames to rows of p >= n frames (zeros behind), `esz` bytes each (2, 4 or 8); dst
+// is 16-byte aligned and p * esz a multiple of 16.
+cudaError_t launch_pad_frames(const void* src, void* dst, int64_t rows, int n, int p, int esz, cudaStream_t st);
+// *fast = contiguous extent of the scan points when they are a flattened grid of at least
+// kProbeMinFast x kProbeMinOuter points (the first index whose x or y differ from point 0, if it
+// divides n_vox), else 0.
+cudaError_t launch_probe_grid(const float* scan, int64_t n_vox, int32_t* fast, cudaStream_t st);
 
 // Power-Doppler epilogue (das_power.cu): out[v] (+)= sum over frames of |in[v][f]|^2.
 cudaError_t launch_power_epilogue(const void* in, float* out, int64_t n_vox, int n_frames, bool cplx, bool accumulate,

@@ -16,6 +16,7 @@
 
 #include "das_launch.cuh"
 #include "das_split.h"
+#include "das_tiles.h"
 #include "mach_b200.h"
 
 #ifndef MACH_B200_NVCC_VERSION
@@ -364,32 +365,48 @@ bool plan_frame_lane(int storage, int interp, uint64_t n_vox, uint32_t n_frames,
     return true;
 }
 
+// A padded copy of the channel data is made when it and its 32-bit offsets stay bounded: at most
+// kPadBytes (what the library's pool keeps between calls), and one launch's worth of samples per
+// transmit.
+constexpr uint64_t kPadBytes = uint64_t{1} << 30;
+
+bool pad_fits(uint32_t n_rx, uint32_t n_samples, uint32_t n_tx, uint32_t padded, int esz) {
+    const uint64_t per_tx = static_cast<uint64_t>(n_rx) * n_samples * padded;
+    if (per_tx == 0 || n_tx == 0 || per_tx >= (uint64_t{1} << 31)) return false;
+    return per_tx * esz <= kPadBytes / n_tx;
+}
+
 // interp < 0: a caller that runs neither the frame-lane nor the ensemble kernel; batch: a
-// persistent batch, which runs the frame-lane kernel but not the ensemble kernel.
+// persistent batch, which runs the frame-lane kernel but not the ensemble kernel; may_pad: the
+// caller can run a lane-voxel job on a copy of its channel data with padded frame rows; probe: the
+// caller can look for the voxel grid on the device.
 Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, const void* channel,
                  bool channel_on_device, const mach_b200_options& o, int interp = -1, bool batch = false,
-                 uint32_t n_rx = 0, uint32_t n_samples = 0) {
+                 uint32_t n_rx = 0, uint32_t n_samples = 0, bool may_pad = false, bool probe = false) {
     Plan p;
     const int esz = static_cast<int>(storage_bytes(storage));
     const int vf = 8 / esz;
+    const bool cplx = (storage & 1) != 0;
     int kind = o.kernel;
-    // Longer ensembles in chunks of 8 frames (one CTA per chunk and tile) of the voxel-per-lane
-    // kernel: rows of 8 frames must be 16-byte vectors and every sample row a multiple of 16
-    // bytes.
-    // (8-frame rows of 32 or more bytes are read with 256-bit loads: 32-byte aligned channel data)
-    const uintptr_t align8 = (8u * esz) % 32u == 0 ? 32 : 16;
-    const bool lane8_ok = n_frames > 16 && n_frames % 8 == 0 && (8u * esz) % 16u == 0 &&
-                          (static_cast<uint64_t>(n_frames) * esz) % 16u == 0 &&
-                          (!channel_on_device || reinterpret_cast<uintptr_t>(channel) % align8 == 0);
-    // Measured on B200 (200-frame Doppler): for 4-byte complex storage (cf16, cbf16, ci16) the
-    // 8-frame chunks beat the ensemble kernel (3.5 vs 5.5 ms); for complex64 and real storage
-    // the ensemble kernel wins.
-    // Measured on B200 (200-frame Doppler): the 8-frame chunks beat the ensemble kernel for
-    // complex storage -- 3.3 vs 5.6 ms (cf16), 4.0 vs 4.8 ms (complex64, 256-bit row loads).
-    if (kind == MACH_B200_KERNEL_AUTO && lane8_ok && (esz == 4 || esz == 8) && (storage & 1) &&
-        grid_matches(o, n_vox)) {
-        kind = MACH_B200_KERNEL_LANE_VOXEL;
-    }
+    // More frames than one lane holds: chunks of 8 complex or 16 real frames (one CTA per chunk and
+    // tile) of the voxel-per-lane kernel.  Its rows must be whole chunks, 32-byte aligned (8 complex
+    // frames of 4 bytes and 16 real ones of 2 are 32 bytes; 256-bit loads).  Real rows of a multiple
+    // of 8 frames run in chunks of 8.  Other frame counts and alignments run on a padded copy
+    // where the caller can make one.
+    const uint32_t fc = cplx ? 8 : 16;
+    const uint32_t padded = (n_frames + fc - 1) / fc * fc;
+    const uintptr_t base = channel_on_device ? reinterpret_cast<uintptr_t>(channel) : 0;
+    const bool rows_ok = n_frames > 8 && padded == n_frames && base % 32 == 0;
+    const bool real8_ok = !cplx && n_frames > 16 && n_frames % 8 == 0 && base % ((8u * esz) % 32u == 0 ? 32 : 16) == 0;
+    const bool pad_ok = may_pad && n_frames > 8 && pad_fits(n_rx, n_samples, n_tx, padded, esz);
+    const bool chunks_ok = rows_ok || real8_ok || pad_ok;
+    // Measured on B200 against the staged kernel: 12 complex64 frames x 3 transmits 619 -> 236 us, 12
+    // float32 frames 464 -> 176 us, 9 int16 pairs 537 -> 237 us (all on padded copies), and against the
+    // ensemble kernel: 200 complex64 frames 4.87 -> 3.67 ms, 64 int16 frames 757 -> 374 us (2-D) and
+    // 64.9 -> 63.4 ms (3-D).  Float32 ensembles of 64 or more frames on a 3-D grid stay with the ensemble
+    // kernel (60.7 ms against 75.6 ms; 2-D, 96 frames: 931 us against 797 us).
+    const bool chunks_first = cplx || esz == 2 || n_frames < 64 || !(grid_matches(o, n_vox) && o.grid_shape[1] > 1);
+    if (kind == MACH_B200_KERNEL_AUTO && chunks_ok && chunks_first) kind = MACH_B200_KERNEL_LANE_VOXEL;
     // Frame-lane kernel: when asked for (measured on B200, the ensemble kernel and the 8-frame
     // chunks stay faster on the 200-frame Doppler job; the autotuner times all three).
     if (interp >= 0 && kind == MACH_B200_KERNEL_FRAME_LANE) {
@@ -410,19 +427,27 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
     // Host channel data is staged into fresh (aligned) device buffers.
     const bool vec_ok =
         n_frames % static_cast<uint32_t>(vf) == 0 && (!channel_on_device || reinterpret_cast<uintptr_t>(channel) % 8 == 0);
-    // 16 frames per sample (32 bytes or more) as 256-bit vectors: 32-byte aligned rows.
-    const bool lane16_ok = n_frames == 16 && (16u * esz) % 32u == 0 &&
-                           (!channel_on_device || reinterpret_cast<uintptr_t>(channel) % 32 == 0);
     if (kind == MACH_B200_KERNEL_AUTO) {
-        kind = (n_frames <= 8 || lane16_ok) ? MACH_B200_KERNEL_LANE_VOXEL
-                                            : (vec_ok ? MACH_B200_KERNEL_STAGED : MACH_B200_KERNEL_WARP);
+        kind = n_frames <= 8 || chunks_ok ? MACH_B200_KERNEL_LANE_VOXEL
+                                          : (vec_ok ? MACH_B200_KERNEL_STAGED : MACH_B200_KERNEL_WARP);
     }
-    if (kind == MACH_B200_KERNEL_LANE_VOXEL && n_frames > 8 && !lane16_ok && !lane8_ok) kind = MACH_B200_KERNEL_WARP;
+    if (kind == MACH_B200_KERNEL_LANE_VOXEL && n_frames > 8 && !chunks_ok) kind = MACH_B200_KERNEL_WARP;
     if (kind == MACH_B200_KERNEL_STAGED && !vec_ok) kind = MACH_B200_KERNEL_WARP;
 
     if (kind == MACH_B200_KERNEL_LANE_VOXEL) {
-        p.lp.kind = n_frames <= 1 ? kKindLaneVoxel1 : (n_frames == 16 ? kKindLaneVoxel16 : kKindLaneVoxelN);
-        if (n_frames > 16) p.lp.kind = kKindLaneVoxel8;  // lane8_ok (checked above)
+        p.lp.kind = n_frames <= 1 ? kKindLaneVoxel1 : kKindLaneVoxelN;
+        if (n_frames > 8) {
+            // Chunks of 16 for complex64 rows that hold them: the arithmetic of a point's delay is
+            // shared by twice the frames.  4-byte complex samples and quadratic taps stay at 8 (16
+            // cost them 128 registers).  Measured on B200, chunks of 8 / 16: complex64 12 frames x 3
+            // transmits 299 / 236 us, 64 frames 339 / 301 us, 192 frames x 5 3.97 / 3.80 ms; FP16
+            // pairs, 192 frames 3.08 / 3.47 ms; complex64 quadratic, 12 frames 311 / 356 us.
+            const bool sixteen = esz == 8 && interp != kQuadratic && padded % 16 == 0;
+            const bool eight = cplx ? !sixteen : (!rows_ok && real8_ok);
+            p.lp.kind = eight ? kKindLaneVoxel8 : kKindLaneVoxel16;
+            p.lp.pad_frames = !rows_ok && !real8_ok ? static_cast<int>(padded) : 0;
+            p.lp.frame_chunks = static_cast<int>((eight && !cplx ? n_frames : padded) / (eight ? 8 : 16));
+        }
         p.lp.passes = static_cast<int>(n_frames);
         p.lp.block = dim3(kLaneVoxelThreads, 1, 1);
         // One-frame jobs split each voxel's elements over 2 or 4 lanes.  Measured on B200: 4
@@ -456,24 +481,27 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
             // Heaviest tiles first (measured on B200: compounding 1.90 -> 1.72 ms, Doppler
             // complex64 4.06 -> 3.84 ms, FP16 2.75 -> 2.48 ms; 3-D 16 frames 67.3 -> 67.8 ms,
             // so 16-frame jobs keep the grid order).
-            p.lp.tile_rev = o.tile_order == 1 ? 1 : (o.tile_order == 2 ? 0 : (n_frames == 16 ? 0 : 1));
+            p.lp.tile_rev = o.tile_order == 1 ? 1 : (o.tile_order == 2 ? 0 : (p.lp.kind == kKindLaneVoxel16 ? 0 : 1));
             p.lp.map_outer = static_cast<int64_t>(n_vox / static_cast<uint64_t>(o.grid_shape[2]));
             const int64_t per_outer = vpc >> lw;
             const int64_t tiles = ((p.lp.map_outer + per_outer - 1) / per_outer) * ((p.lp.map_fast + wf - 1) / wf);
             p.lp.grid = dim3(static_cast<unsigned>(tiles), 1, 1);
         }
-        if (p.lp.kind == kKindLaneVoxel8) {  // the 8-frame chunks of a tile run on consecutive CTAs
-            p.lp.frame_chunks = static_cast<int>(n_frames / 8);
-            p.lp.grid.x *= static_cast<unsigned>(p.lp.frame_chunks);
+        else if (probe && n_frames > 8) {
+            p.lp.probe_grid = true;
+            p.lp.map_wlog = wf == 1 ? 0 : (wf == 2 ? 1 : (wf == 4 ? 2 : (wf == 8 ? 3 : 4)));
+            p.lp.tile_rev = p.lp.kind == kKindLaneVoxel16 ? 0 : 1;
+            p.lp.grid = dim3(static_cast<unsigned>(probed_tiles(static_cast<int64_t>(n_vox), vpc, wf)), 1, 1);
         }
+        if (p.lp.frame_chunks > 1) p.lp.grid.x *= static_cast<unsigned>(p.lp.frame_chunks);  // consecutive CTAs
         // Element blocks: one launch per block of elements whose channel data (all transmits)
         // fits in L2 with room to spare.  Automatic for 16-frame jobs above 126 MB of channel
         // data (3-D: every CTA sweeps every (transmit, element) row set, and CTAs that drift apart
         // evict each other's rows; measured DRAM reads were 70x the channel data in one launch).
         {
-            const uint64_t per_elem = static_cast<uint64_t>(n_tx) * n_samples * n_frames * esz;
+            const uint64_t per_elem = static_cast<uint64_t>(n_tx) * n_samples * std::max<uint32_t>(n_frames, p.lp.pad_frames) * esz;
             int eb = o.element_block;
-            if (eb == 0 && n_frames == 16 && per_elem > 0 &&
+            if (eb == 0 && p.lp.kind == kKindLaneVoxel16 && per_elem > 0 &&
                 per_elem * n_rx > (uint64_t{126} << 20) && !batch) {
                 eb = static_cast<int>(std::max<uint64_t>(32, ((uint64_t{80} << 20) / per_elem) / 32 * 32));
             }
@@ -751,6 +779,7 @@ DasArgs make_args(const float* rx_coords_m, const float* scan_coords_m, uint64_t
     a.e_end = a.n_rx;
     a.n_samples = static_cast<int32_t>(n_samples);
     a.n_frames = static_cast<int32_t>(n_frames);
+    a.row_frames = a.n_frames;
     a.row_stride = static_cast<int64_t>(n_samples) * n_frames;
     a.inv_c = 1.0f / sound_speed_m_s;  // kernel.cu:750, FP32 on the host
     a.fs = sampling_freq_hz;
@@ -815,7 +844,7 @@ int compound_impl(int32_t storage, const void* channel_data, const float* rx_coo
                   const float* tx_wave_arrivals_s, void* out, uint32_t n_tx, uint32_t n_rx, uint32_t n_samples,
                   uint64_t n_scan, uint32_t n_frames, float f_number, float rx_start_s, float sampling_freq_hz,
                   float sound_speed_m_s, float modulation_freq_hz, float tukey_alpha, int32_t interp_type,
-                  float channel_scale, cudaStream_t stream, const mach_b200_options& opt) {
+                  float channel_scale, cudaStream_t stream, const mach_b200_options& opt, bool probe_grid = false) {
     if (opt.flags & MACH_B200_FLAG_POWER_DOPPLER) {
         return power_impl(storage, channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out, n_tx, n_rx,
                           n_samples, n_scan, n_frames, f_number, rx_start_s, sampling_freq_hz, sound_speed_m_s,
@@ -854,8 +883,21 @@ int compound_impl(int32_t storage, const void* channel_data, const float* rx_coo
                           rx_start_s, sampling_freq_hz, sound_speed_m_s, modulation_freq_hz, tukey_alpha,
                           channel_scale, cplx, flags);
     const bool overwrite = (flags & MACH_B200_FLAG_OVERWRITE) != 0u || r_out != kOnDevice;
-    Plan plan = plan_launch(storage, n_scan, n_frames, n_tx, channel_data, r_ch == kOnDevice, opt, interp_type, false,
-                            n_rx, n_samples);
+    const bool all_device = r_ch == kOnDevice && r_rx == kOnDevice && r_scan == kOnDevice && r_arr == kOnDevice &&
+                            r_out == kOnDevice;
+    // A job of device buffers may run on a padded copy of its channel data and, where the caller
+    // gives no voxel grid to go by, look for it on the device.
+    auto make_plan = [&](bool may_pad) {
+        return plan_launch(storage, n_scan, n_frames, n_tx, channel_data, r_ch == kOnDevice, opt, interp_type, false,
+                           n_rx, n_samples, may_pad && all_device && need_channel, probe_grid && all_device);
+    };
+    Plan plan = make_plan(true);
+    DeviceBuffer padded, probed;
+    if (plan.lp.pad_frames > 0 &&
+        padded.alloc(static_cast<size_t>(n_tx) * n_rx * n_samples * plan.lp.pad_frames * esz, stream) != cudaSuccess) {
+        cudaGetLastError();  // no room for the copy: the kernels that read the rows as they are
+        plan = make_plan(false);
+    }
     plan.st.status = dev->status;
     a.frame_passes = plan.lp.passes;
     a.tx_chunk = plan.lp.tx_chunk;
@@ -865,10 +907,23 @@ int compound_impl(int32_t storage, const void* channel_data, const float* rx_coo
     a.map_outer = plan.lp.map_outer;
     a.frame_chunks = plan.lp.frame_chunks;
 
-    const bool all_device = r_ch == kOnDevice && r_rx == kOnDevice && r_scan == kOnDevice && r_arr == kOnDevice &&
-                            r_out == kOnDevice;
     if (all_device) {
         a.channel = channel_data;
+        if (plan.lp.pad_frames > 0) {
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            MACH_B200_CUDA_TRY(launch_pad_frames(channel_data, padded.ptr, static_cast<int64_t>(n_tx) * n_rx * n_samples,
+                                                 static_cast<int>(n_frames), plan.lp.pad_frames, static_cast<int>(esz),
+                                                 stream));
+            a.channel = padded.ptr;
+            a.row_frames = plan.lp.pad_frames;
+            a.row_stride = static_cast<int64_t>(n_samples) * plan.lp.pad_frames;
+        }
+        if (plan.lp.probe_grid) {
+            MACH_B200_CUDA_TRY(probed.alloc(sizeof(int32_t), stream));
+            g_launches.fetch_add(1, std::memory_order_relaxed);
+            MACH_B200_CUDA_TRY(launch_probe_grid(scan_coords_m, a.n_vox, static_cast<int32_t*>(probed.ptr), stream));
+            a.probed_fast = static_cast<const int32_t*>(probed.ptr);
+        }
         a.arrivals = tx_wave_arrivals_s;
         a.out = out;
         a.n_tx = static_cast<int32_t>(need_channel ? n_tx : 0);
@@ -1129,7 +1184,8 @@ int power_impl(int32_t storage, const void* channel_data, const float* rx_coords
 
     // ---- fused: the ensemble / frame-lane kernel adds |x|^2 of each frame block into out
     if (all_device && need_channel) {
-        Plan plan = plan_launch(storage, n_scan, n_frames, n_tx, channel_data, true, opt, interp_type);
+        Plan plan = plan_launch(storage, n_scan, n_frames, n_tx, channel_data, true, opt, interp_type, false, n_rx,
+                                n_samples, true);
         const int64_t per_tx = static_cast<int64_t>(n_rx) * n_samples * n_frames;
         if ((plan.ensemble || plan.frame_lane) && per_tx * n_tx < (int64_t{1} << 31)) {
             plan.st.status = dev->status;
@@ -1710,7 +1766,7 @@ int mach_b200_beamform_f32(const float* channel_data, const float* rx_coords_m, 
                            float tukey_alpha, int32_t interp_type) {
     return compound_impl(kF32, channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out, 1u, n_rx,
                          n_samples, n_scan, n_frames, f_number, rx_start_s, sampling_freq_hz, sound_speed_m_s,
-                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(0u));
+                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(0u), true);
 }
 
 int mach_b200_beamform_c64(const void* channel_data, const float* rx_coords_m, const float* scan_coords_m,
@@ -1720,7 +1776,7 @@ int mach_b200_beamform_c64(const void* channel_data, const float* rx_coords_m, c
                            float tukey_alpha, int32_t interp_type) {
     return compound_impl(kC64, channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out, 1u, n_rx,
                          n_samples, n_scan, n_frames, f_number, rx_start_s, sampling_freq_hz, sound_speed_m_s,
-                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(0u));
+                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(0u), true);
 }
 
 int mach_b200_beamform_compound(int32_t storage, const void* channel_data, const float* rx_coords_m,
