@@ -298,6 +298,33 @@ int hilbert_plan(int n, int* radix, int max_stages);
 // resident CTAs.
 cudaError_t launch_hilbert(int src_code, int dst_code, const HilbertArgs& g, size_t smem, cudaStream_t st);
 
+// In-place form for contiguous columns (das_hilbert_cols.cu): digit j of the index has radix[j], buffer
+// stride stride[j], low[j] indexes below it and frequency weight weight[j]; r_* are reciprocals.
+constexpr int kHilColsMaxStages = 6;
+constexpr int kHilColsMaxPairsLog2 = 4;
+struct HilbertColsArgs {
+    const void* src;
+    void* dst;
+    int src_code, dst_code;
+    int n, m;
+    int radix[kHilColsMaxStages], stride[kHilColsMaxStages], low[kHilColsMaxStages], weight[kHilColsMaxStages],
+        items[kHilColsMaxStages];
+    float r_radix[kHilColsMaxStages], r_low[kHilColsMaxStages], r_items[kHilColsMaxStages];
+    int twiddles;    // float2 of all stages' tables
+    int pairs_log2;  // a CTA takes 2^pairs_log2 column pairs
+    int pair_size;   // float2 of one pair's buffer
+    int pair_vec;    // 1: the two columns of a float32 pair are adjacent, 8-byte aligned
+    float inv_n, scale;
+    int64_t n_cols;  // column c = (c / n1, c % n1)
+    int64_t n1;
+    int64_t src_stride[2], dst_stride[2];  // of c % n1 and c / n1
+    int64_t src_sample;                    // between samples of a source column; destination columns are contiguous
+};
+// Radices, strides and pairs per CTA for length n; false when n is no product of the radices.
+bool hilbert_cols_plan(int n, HilbertColsArgs& g);
+size_t hilbert_cols_smem(const HilbertColsArgs& g);
+cudaError_t launch_hilbert_cols(const HilbertColsArgs& g, cudaStream_t st);
+
 // Transmit arrivals of a plane (model 1) or spherical (model 2) wave table (das_transmit.cu):
 // out[t][v] for t < n_tx, v < n_scan; params [n_tx][8] FP64, scan [n_scan][3] FP32, all
 // device memory.

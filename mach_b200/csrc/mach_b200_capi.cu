@@ -1372,7 +1372,32 @@ int hilbert_impl(int32_t src_storage, const void* src, int32_t src_layout, int32
     }
     g.dst = dst;
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    MACH_B200_CUDA_TRY(launch_hilbert(src_storage, dst_storage, g, smem, stream));
+    // Contiguous destination columns of a length that its radices divide: the in-place kernel.  With
+    // several frames per sample the out-of-place kernel stays: it walks a group of up to 16
+    // columns column-fastest, so that its writes are contiguous too.
+    HilbertColsArgs h{};
+    const bool planned = F == 1 && hilbert_cols_plan(g.n, h);
+    h.pair_vec = src_storage == kF32 && src_layout == MACH_B200_LAYOUT_ACQUISITION && n_cols % 2 == 0 &&
+                 reinterpret_cast<uintptr_t>(g.src) % 8 == 0;
+    if (planned && hilbert_cols_smem(h) > static_cast<size_t>(max_smem) - 4096) h.pair_vec = 0;
+    if (planned && hilbert_cols_smem(h) <= static_cast<size_t>(max_smem) - 4096) {
+        h.src = g.src;
+        h.dst = dst;
+        h.src_code = src_storage;
+        h.dst_code = dst_storage;
+        h.inv_n = g.inv_n;
+        h.scale = scale;
+        h.n_cols = n_cols;
+        h.n1 = g.n1;
+        for (int k = 0; k < 2; ++k) {
+            h.src_stride[k] = g.src_stride[k + 1];
+            h.dst_stride[k] = g.dst_stride[k + 1];
+        }
+        h.src_sample = g.src_sample;
+        MACH_B200_CUDA_TRY(launch_hilbert_cols(h, stream));
+    } else {
+        MACH_B200_CUDA_TRY(launch_hilbert(src_storage, dst_storage, g, smem, stream));
+    }
     if (r_src != kOnDevice || !(flags & MACH_B200_FLAG_ASYNC)) MACH_B200_CUDA_TRY(cudaStreamSynchronize(stream));
     return MACH_B200_OK;
 }
