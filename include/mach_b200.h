@@ -74,6 +74,9 @@ extern "C" {
                                            frames of |beamformed value|^2 (the step after the beamformer
                                            in mach's examples/doppler.py:252), fused into the kernel where
                                            it can be; only the compound / _ex entry points take it */
+#define MACH_B200_FLAG_PROBE_GRID 16u /* without a grid_shape, multi-frame jobs of device buffers look for the
+                                         voxel grid on the device (one small kernel) and tile by it, as the
+                                         single-transmit entry points do; never changes a sum */
 
 /* Kernel families (mach_b200_options.kernel). */
 #define MACH_B200_KERNEL_AUTO 0

@@ -111,6 +111,7 @@ FLAG_ASYNC = 1
 FLAG_OVERWRITE = 2
 FLAG_SPLIT_DELAY = 4
 FLAG_POWER_DOPPLER = 8
+FLAG_PROBE_GRID = 16
 
 STORAGE_CODES = {"f32": 0, "c64": 1, "f16": 2, "cf16": 3, "bf16": 4, "cbf16": 5, "i16": 6, "ci16": 7}
 
@@ -274,6 +275,19 @@ def beamform(
     rc = fn(ch.ptr, rx.ptr, scan.ptr, tx.ptr, o.ptr, n_rx, n_samples, n_vox, n_frames, float(f_number),
             float(rx_start_s), float(sampling_freq_hz), float(sound_speed_m_s), float(modulation_freq_hz),
             float(tukey_alpha), int(interp_type))
+    _raise_for(rc)
+
+
+def beamform_tensors(channel, rx, scan, arrivals, out, n_rx: int, n_samples: int, n_vox: int, n_frames: int,
+                     f_number: float, rx_start_s: float, sampling_freq_hz: float, sound_speed_m_s: float,
+                     modulation_freq_hz: float, tukey_alpha: float, interp_type: int, overwrite: bool) -> None:
+    """:func:`beamform` for checked contiguous CUDA torch tensors: the same job on the same (legacy
+    default) stream, without the array descriptions.  ``overwrite``: ``out`` need not be cleared."""
+    rc = _lib.mach_b200_beamform_compound(
+        1 if channel.is_complex() else 0, channel.data_ptr(), rx.data_ptr(), scan.data_ptr(), arrivals.data_ptr(),
+        out.data_ptr(), 1, n_rx, n_samples, n_vox, n_frames, float(f_number), float(rx_start_s),
+        float(sampling_freq_hz), float(sound_speed_m_s), float(modulation_freq_hz), float(tukey_alpha),
+        int(interp_type), 1.0, None, FLAG_PROBE_GRID | (FLAG_OVERWRITE if overwrite else 0))
     _raise_for(rc)
 
 

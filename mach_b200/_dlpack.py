@@ -23,7 +23,7 @@ class NullView:
     ptr = 0
 
 
-@dataclass
+@dataclass(slots=True)
 class ArrayView:
     ptr: int
     shape: tuple[int, ...]
@@ -119,22 +119,16 @@ def _from_capsule(obj: Any) -> ArrayView:
     )
 
 
+_TORCH_DTYPE_NAMES: dict[Any, str] = {}  # torch dtype -> name, filled as dtypes are met
+
+
 def _torch_view(t: Any) -> ArrayView:
-    dtype = str(t.dtype).replace("torch.", "")
-    if dtype == "complex32":
-        dtype = "complex32"
-    dev = t.device
-    return ArrayView(
-        ptr=int(t.data_ptr()),
-        shape=tuple(int(d) for d in t.shape),
-        strides=tuple(int(s) for s in t.stride()),
-        dtype=dtype,
-        itemsize=int(t.element_size()),
-        device_type=CUDA if dev.type == "cuda" else CPU,
-        device_id=int(dev.index or 0) if dev.type == "cuda" else 0,
-        writeable=True,
-        owner=t,
-    )
+    dtype = _TORCH_DTYPE_NAMES.get(t.dtype)
+    if dtype is None:
+        dtype = _TORCH_DTYPE_NAMES[t.dtype] = str(t.dtype).replace("torch.", "")
+    cuda = t.is_cuda
+    return ArrayView(t.data_ptr(), tuple(t.shape), t.stride(), dtype, t.element_size(), CUDA if cuda else CPU,
+                     (t.device.index or 0) if cuda else 0, True, t)
 
 
 def _numpy_view(a: np.ndarray) -> ArrayView:
@@ -152,8 +146,15 @@ def _numpy_view(a: np.ndarray) -> ArrayView:
     )
 
 
+_IS_TORCH: dict[type, bool] = {}  # by type, filled as types are met
+
+
 def is_torch(x: Any) -> bool:
-    return type(x).__module__.startswith("torch")
+    t = type(x)
+    known = _IS_TORCH.get(t)
+    if known is None:
+        known = _IS_TORCH[t] = t.__module__.startswith("torch")
+    return known
 
 
 def view(x: Any) -> ArrayView:

@@ -844,7 +844,7 @@ int compound_impl(int32_t storage, const void* channel_data, const float* rx_coo
                   const float* tx_wave_arrivals_s, void* out, uint32_t n_tx, uint32_t n_rx, uint32_t n_samples,
                   uint64_t n_scan, uint32_t n_frames, float f_number, float rx_start_s, float sampling_freq_hz,
                   float sound_speed_m_s, float modulation_freq_hz, float tukey_alpha, int32_t interp_type,
-                  float channel_scale, cudaStream_t stream, const mach_b200_options& opt, bool probe_grid = false) {
+                  float channel_scale, cudaStream_t stream, const mach_b200_options& opt) {
     if (opt.flags & MACH_B200_FLAG_POWER_DOPPLER) {
         return power_impl(storage, channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out, n_tx, n_rx,
                           n_samples, n_scan, n_frames, f_number, rx_start_s, sampling_freq_hz, sound_speed_m_s,
@@ -889,7 +889,7 @@ int compound_impl(int32_t storage, const void* channel_data, const float* rx_coo
     // gives no voxel grid to go by, look for it on the device.
     auto make_plan = [&](bool may_pad) {
         return plan_launch(storage, n_scan, n_frames, n_tx, channel_data, r_ch == kOnDevice, opt, interp_type, false,
-                           n_rx, n_samples, may_pad && all_device && need_channel, probe_grid && all_device);
+                           n_rx, n_samples, may_pad && all_device && need_channel, (flags & MACH_B200_FLAG_PROBE_GRID) != 0u && all_device);
     };
     Plan plan = make_plan(true);
     DeviceBuffer padded, probed;
@@ -1791,7 +1791,7 @@ int mach_b200_beamform_f32(const float* channel_data, const float* rx_coords_m, 
                            float tukey_alpha, int32_t interp_type) {
     return compound_impl(kF32, channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out, 1u, n_rx,
                          n_samples, n_scan, n_frames, f_number, rx_start_s, sampling_freq_hz, sound_speed_m_s,
-                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(0u), true);
+                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(MACH_B200_FLAG_PROBE_GRID));
 }
 
 int mach_b200_beamform_c64(const void* channel_data, const float* rx_coords_m, const float* scan_coords_m,
@@ -1801,7 +1801,7 @@ int mach_b200_beamform_c64(const void* channel_data, const float* rx_coords_m, c
                            float tukey_alpha, int32_t interp_type) {
     return compound_impl(kC64, channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out, 1u, n_rx,
                          n_samples, n_scan, n_frames, f_number, rx_start_s, sampling_freq_hz, sound_speed_m_s,
-                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(0u), true);
+                         modulation_freq_hz, tukey_alpha, interp_type, 1.0f, nullptr, default_options(MACH_B200_FLAG_PROBE_GRID));
 }
 
 int mach_b200_beamform_compound(int32_t storage, const void* channel_data, const float* rx_coords_m,

@@ -25,6 +25,10 @@ def _current_stream(x: Any) -> int:
     if _dlpack.is_torch(x) and x.device.type == "cuda":
         import torch
 
+        index = x.device.index
+        raw = getattr(torch._C, "_cuda_getCurrentRawStream", None)  # without building a Stream object
+        if raw is not None and index is not None:
+            return int(raw(index))
         return int(torch.cuda.current_stream(x.device).cuda_stream)
     return 0
 
@@ -162,7 +166,12 @@ def _compound(channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out,
     n_points = int(scan_coords_m.shape[0])
     output_dtype = xp.complex64 if is_complex and not power else xp.float32
     out_shape = (n_points,) if power else (n_points, n_frames)
-    if out is None:
+    fresh = False
+    if out is None and ch.on_cuda and _dlpack.is_torch(channel_data):
+        # a result of our own on the GPU: written by the call, not cleared and added to
+        fresh = True
+        out = channel_data.new_empty(out_shape, dtype=output_dtype)
+    elif out is None:
         out = xp.zeros(out_shape, dtype=output_dtype, like=channel_data)
     elif out.dtype != output_dtype:
         raise ValueError(f"Output array dtype {out.dtype} doesn't match expected {output_dtype}")
@@ -201,6 +210,8 @@ def _compound(channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out,
         flags |= _cuda_impl.FLAG_SPLIT_DELAY
     if power:
         flags |= _cuda_impl.FLAG_POWER_DOPPLER
+    if fresh:
+        flags |= _cuda_impl.FLAG_OVERWRITE
     if grid_shape is None:
         grid_shape = _grid.detect(scan_coords_m)
         if (kernel == "auto" and not (window_rows or lanes_per_voxel or tx_chunk or tile_fast or frame_slots
