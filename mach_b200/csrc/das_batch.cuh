@@ -9,6 +9,7 @@
 // transmit counts share the launch; the GPU stays full until the last item.
 #pragma once
 
+#include "das_frame_group.cuh"
 #include "das_frame_lane.cuh"
 #include "das_lane_voxel.cuh"
 #include "das_staged.cuh"
@@ -76,6 +77,26 @@ __global__ void __launch_bounds__(kLaneVoxelThreads, lane_voxel_ctas<S, INTERP, 
         } else {
             lane_voxel_tile<S, INTERP, NF, SPLIT, CS>(s_args, s_local, smem_words);
         }
+    }
+}
+
+// (the arguments are read from shared memory here: one or two CTAs of registers more than the
+// per-job kernel)
+template <int S, int INTERP, int LF, bool SPLIT>
+__global__ void __launch_bounds__(kLaneVoxelThreads, frame_group_ctas<S, INTERP, LF>() - (LF == 4 ? 2 : 1))
+    das_frame_group_persistent(const BatchHeader* __restrict__ hdr, const BatchJob* __restrict__ jobs,
+                               const int64_t* __restrict__ item_begin, unsigned long long* counter) {
+    extern __shared__ float smem_words[];
+    __shared__ DasArgs s_args;
+    __shared__ int s_job;
+    __shared__ int64_t s_local;
+    int cursor = 0;
+    while (next_item(hdr, item_begin, counter, cursor, &s_job, &s_local)) {
+        copy_words(&s_args, &jobs[s_job].a);
+        __syncthreads();
+        const int64_t tile = s_local / s_args.frame_chunks;
+        frame_group_tile<S, INTERP, LF, SPLIT>(s_args, tile, smem_words,
+                                               static_cast<int>(s_local - tile * s_args.frame_chunks));
     }
 }
 

@@ -140,7 +140,8 @@ struct DasArgs {
     // deepest first for a depth-fastest scan, whose wide apertures make them the heaviest), so the
     // CTAs that start last take light tiles; 0: grid order (outer-major).
     int32_t tile_rev;
-    int32_t frame_chunks;   // lane-voxel chunks of 8 or 16 frames: CTA b takes tile b / frame_chunks, chunk b % frame_chunks
+    int32_t frame_chunks;   // lane-voxel and frame-group kernels: CTA b takes tile b / frame_chunks, chunk b % frame_chunks
+    int32_t frame_first;    // first frame of chunk 0
     int32_t row_frames;     // lane-voxel kernels: frames stored per sample (n_frames; more in a padded copy)
     // Lane-voxel kernels without a known grid: device word with the contiguous extent that
     // das_probe_grid_kernel found (0: none), read instead of map_fast; nullptr otherwise.

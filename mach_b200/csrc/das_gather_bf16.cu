@@ -13,4 +13,6 @@ template cudaError_t launch_das_ensemble<kBF16>(const DasArgs&, const StagedArgs
 template cudaError_t launch_das_frame_lane<kBF16>(const DasArgs&, const FrameLaneArgs&, int, const LaunchPlan&,
                                                 cudaStream_t);
 template cudaError_t launch_frame_lane_persistent<kBF16>(int, int, bool, const PersistentLaunch&, cudaStream_t);
+template cudaError_t launch_frame_group_persistent<kBF16>(int, int, bool, const PersistentLaunch&,
+                                                               cudaStream_t);
 }  // namespace mach_b200

@@ -13,4 +13,6 @@ template cudaError_t launch_das_ensemble<kC64>(const DasArgs&, const StagedArgs&
 template cudaError_t launch_das_frame_lane<kC64>(const DasArgs&, const FrameLaneArgs&, int, const LaunchPlan&,
                                                 cudaStream_t);
 template cudaError_t launch_frame_lane_persistent<kC64>(int, int, bool, const PersistentLaunch&, cudaStream_t);
+template cudaError_t launch_frame_group_persistent<kC64>(int, int, bool, const PersistentLaunch&,
+                                                               cudaStream_t);
 }  // namespace mach_b200

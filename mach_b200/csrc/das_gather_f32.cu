@@ -13,4 +13,6 @@ template cudaError_t launch_das_ensemble<kF32>(const DasArgs&, const StagedArgs&
 template cudaError_t launch_das_frame_lane<kF32>(const DasArgs&, const FrameLaneArgs&, int, const LaunchPlan&,
                                                 cudaStream_t);
 template cudaError_t launch_frame_lane_persistent<kF32>(int, int, bool, const PersistentLaunch&, cudaStream_t);
+template cudaError_t launch_frame_group_persistent<kF32>(int, int, bool, const PersistentLaunch&,
+                                                               cudaStream_t);
 }  // namespace mach_b200

@@ -203,11 +203,7 @@ struct FramePieces {
     // different sample rows, often at the same offset of a 128-byte line; starting some lanes with
     // another piece spreads the four over the line's banks (200-frame complex64 Doppler on B200:
     // L1 data pipe 94 -> 72 % busy, 3.77 -> 3.67 ms; load latency bounds it now).
-    __device__ static __forceinline__ int first(int lane) {
-        if constexpr (kCount == 2) return (lane >> 1) & 1;
-        if constexpr (kCount == 4) return lane & 3;
-        return 0;
-    }
+    __device__ static __forceinline__ int first(int lane) { return kCount == 2 ? (lane >> 1) & 1 : 0; }
 };
 
 // Load the NF frames of one sample (NF * sizeof(T) is a multiple of 16 bytes), piece by piece from
@@ -518,7 +514,7 @@ __device__ __forceinline__ void lane_voxel_tile(const DasArgs& a, int64_t tile, 
     // Frames stored per sample row (n_frames, or more in a padded copy), and this CTA's first frame:
     // vector jobs with more frames than NF run in chunks of NF frames.
     const int fstride = a.row_frames;
-    const int f0 = NF >= 2 ? chunk * NF : 0;
+    const int f0 = NF >= 2 ? a.frame_first + chunk * NF : 0;
 
     float vx = 0.f, vy = 0.f, vz = 0.f;
     if (vox_ok) {
@@ -1083,11 +1079,11 @@ __device__ __forceinline__ float2 gather_taps(const typename Storage<S>::T* row,
 }
 
 // CTAs per SM that the register budget is cut for, from the state a point keeps live: 16 frames of
-// 16-bit real samples fit 72 registers, of float32 96, of complex samples 128; 8 complex64 frames 72
-// (quadratic: three rows in flight, 96); the other kernels 64.
+// 16-bit real samples fit 72 registers, of float32 96; 8 complex64 frames 72 (quadratic: three
+// rows in flight, 96); the other kernels 64.
 template <int S, int INTERP, int NF>
 constexpr int lane_voxel_ctas() {
-    if (NF == 16) return Storage<S>::kComplex ? 4 : (S == kF32 ? 5 : 7);
+    if (NF == 16) return S == kF32 ? 5 : 7;
     if (NF == 8 && S == kC64) return INTERP == kQuadratic ? 5 : 7;
     return 8;
 }

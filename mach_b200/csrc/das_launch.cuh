@@ -5,19 +5,13 @@
 
 #include "das_batch.cuh"
 #include "das_ensemble.cuh"
+#include "das_frame_group.cuh"
 #include "das_frame_lane.cuh"
 #include "das_gather.cuh"
 #include "das_lane_voxel.cuh"
 #include "das_staged.cuh"
 
 namespace mach_b200 {
-
-// Instances of the 16-frame lane-voxel kernels: the plans that ask for them (plan_launch) are real
-// storage and complex64 with one or two taps.
-template <int S, int I>
-constexpr bool lane_voxel_has16() {
-    return !Storage<S>::kComplex || (S == kC64 && I != kQuadratic);
-}
 
 enum KernelKind : int {
     kKindLaneVoxel1 = 0,   // das_lane_voxel_kernel, exactly one frame
@@ -29,11 +23,13 @@ enum KernelKind : int {
     kKindEnsemble = 6,     // das_ensemble_kernel, windows in tensor memory, lanes = frames
     kKindLaneVoxel8 = 7,   // das_lane_voxel_kernel, chunks of 8 frames (grid.y) of a longer ensemble
     kKindFrameLane = 8,    // das_frame_lane_kernel, lanes = frames, rows reused along voxel runs
+    kKindFrameGroup = 9,   // das_frame_group_kernel, 2 or 4 lanes per voxel, 8 complex frames each
 };
 
 struct LaunchPlan {
     int kind;
-    int lanes_per_voxel;  // staged kernel: 4, 8, 16 or 32; one-frame lane-voxel kernel: 1, 2 or 4 lanes per voxel
+    int lanes_per_voxel;  // staged kernel: 4, 8, 16 or 32; one-frame lane-voxel kernel: 1, 2 or 4 lanes per voxel;
+                          // frame-group kernel: 2 or 4
     int passes;       // frames per lane (multi-frame kernels)
     int tx_chunk;     // arrivals staged per pass (lane-voxel kernels)
     dim3 grid;
@@ -43,7 +39,8 @@ struct LaunchPlan {
     int map_wlog;
     int64_t map_outer;
     int tile_rev;       // lane-voxel kernels on a grid: far end of the contiguous axis first (DasArgs::tile_rev)
-    int frame_chunks;   // lane-voxel chunks of 8 or 16 frames per tile (DasArgs::frame_chunks)
+    int frame_chunks;   // lane-voxel and frame-group kernels: chunks per tile (DasArgs::frame_chunks)
+    int frame_first;    // first frame of chunk 0 (DasArgs::frame_first)
     int pad_frames;     // lane-voxel kernels: frames per sample of the padded copy to run on, 0 = none
     bool probe_grid;    // lane-voxel kernels: tile by the extent that a probe of the scan points finds
     int element_block;  // lane-voxel kernels: elements per launch (0 = all), so that one launch's
@@ -109,6 +106,11 @@ cudaError_t launch_das(const DasArgs& a, int interp, const LaunchPlan& p, cudaSt
         if (a.split) das_lane_voxel_kernel<S, I, 1, true, CS><<<p.grid, p.block, p.smem, stream>>>(a);   \
         else das_lane_voxel_kernel<S, I, 1, false, CS><<<p.grid, p.block, p.smem, stream>>>(a);          \
     } while (0)
+#define MACH_B200_FG(I, LF)                                                                          \
+    do {                                                                                             \
+        if (a.split) das_frame_group_kernel<S, I, LF, true><<<p.grid, p.block, p.smem, stream>>>(a); \
+        else das_frame_group_kernel<S, I, LF, false><<<p.grid, p.block, p.smem, stream>>>(a);        \
+    } while (0)
 #define MACH_B200_WG(I, L, P) das_gather_kernel<S, I, L, P><<<p.grid, p.block, 0, stream>>>(a)
 #define MACH_B200_KINDS(I)                                   \
     switch (p.kind) {                                        \
@@ -119,9 +121,15 @@ cudaError_t launch_das(const DasArgs& a, int interp, const LaunchPlan& p, cudaSt
             break;                                           \
         case kKindLaneVoxelN: MACH_B200_LV(I, 0); break;     \
         case kKindLaneVoxel16:                               \
-            if constexpr (lane_voxel_has16<S, I>()) MACH_B200_LV(I, 16); \
+            if constexpr (!Storage<S>::kComplex) MACH_B200_LV(I, 16); \
             break;                                           \
         case kKindLaneVoxel8: MACH_B200_LV(I, 8); break;     \
+        case kKindFrameGroup:                                \
+            if constexpr (Storage<S>::kComplex) {            \
+                if (p.lanes_per_voxel == 4) MACH_B200_FG(I, 4); \
+                else MACH_B200_FG(I, 2);                     \
+            }                                                \
+            break;                                           \
         case kKindWarpHalf: MACH_B200_WG(I, 16, 4); break;   \
         default: MACH_B200_WG(I, 32, 8); break;              \
     }
@@ -132,6 +140,7 @@ cudaError_t launch_das(const DasArgs& a, int interp, const LaunchPlan& p, cudaSt
     }
 #undef MACH_B200_KINDS
 #undef MACH_B200_WG
+#undef MACH_B200_FG
 #undef MACH_B200_LV_CS
 #undef MACH_B200_LV
     return cudaGetLastError();
@@ -202,7 +211,7 @@ cudaError_t launch_lane_voxel_persistent(int interp, int frame_class, bool split
         case 12: MACH_B200_PLV(I, 1, 2);            \
         case 14: MACH_B200_PLV(I, 1, 4);            \
         case 16:                                    \
-            if constexpr (lane_voxel_has16<S, I>()) {MACH_B200_PLV(I, 16, 1);} \
+            if constexpr (!Storage<S>::kComplex) {MACH_B200_PLV(I, 16, 1);} \
             return cudaErrorInvalidValue;           \
         case 8: MACH_B200_PLV(I, 8, 1);             \
         default: MACH_B200_PLV(I, 0, 1);            \
@@ -214,6 +223,28 @@ cudaError_t launch_lane_voxel_persistent(int interp, int frame_class, bool split
     }
 #undef MACH_B200_PLV_NF
 #undef MACH_B200_PLV
+}
+
+// Frame-group family: variant = lanes per voxel (2, 4); complex storage.
+template <int S>
+cudaError_t launch_frame_group_persistent(int interp, int lanes, bool split, const PersistentLaunch& pl,
+                                          cudaStream_t stream) {
+    if constexpr (Storage<S>::kComplex) {
+#define MACH_B200_PFG(I, LF)                                                                                    \
+    return split ? launch_persistent(das_frame_group_persistent<S, I, LF, true>, kLaneVoxelThreads, pl, stream) \
+                 : launch_persistent(das_frame_group_persistent<S, I, LF, false>, kLaneVoxelThreads, pl, stream)
+#define MACH_B200_PFG_LF(I)          \
+    if (lanes == 4) MACH_B200_PFG(I, 4); \
+    MACH_B200_PFG(I, 2)
+        switch (interp) {
+            case kNearest: MACH_B200_PFG_LF(kNearest);
+            case kLinear: MACH_B200_PFG_LF(kLinear);
+            default: MACH_B200_PFG_LF(kQuadratic);
+        }
+#undef MACH_B200_PFG_LF
+#undef MACH_B200_PFG
+    }
+    return cudaErrorInvalidValue;
 }
 
 // Frame-lane family: variant = J (1, 2, 4).

@@ -39,7 +39,9 @@ namespace mach_b200 {
                                                                 cudaStream_t);                               \
     extern template cudaError_t launch_staged_persistent<S>(int, int, const PersistentLaunch&, cudaStream_t); \
     extern template cudaError_t launch_frame_lane_persistent<S>(int, int, bool, const PersistentLaunch&,    \
-                                                                cudaStream_t);
+                                                                cudaStream_t);                               \
+    extern template cudaError_t launch_frame_group_persistent<S>(int, int, bool, const PersistentLaunch&,   \
+                                                                 cudaStream_t);
 MACH_B200_EXTERN(kF32)
 MACH_B200_EXTERN(kC64)
 MACH_B200_EXTERN(kF16)
@@ -208,6 +210,8 @@ constexpr int kMaxTxChunkSplit = 32;
 
 struct Plan {
     LaunchPlan lp{};
+    LaunchPlan rest{};      // second launch of the frames that lp leaves (lane-voxel family)
+    bool has_rest = false;
     StagedArgs st{};
     EnsembleArgs ea{};
     FrameLaneArgs fl{};
@@ -435,81 +439,96 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
     if (kind == MACH_B200_KERNEL_STAGED && !vec_ok) kind = MACH_B200_KERNEL_WARP;
 
     if (kind == MACH_B200_KERNEL_LANE_VOXEL) {
-        p.lp.kind = n_frames <= 1 ? kKindLaneVoxel1 : kKindLaneVoxelN;
-        if (n_frames > 8) {
-            // Chunks of 16 for complex64 rows that hold them: the arithmetic of a point's delay is
-            // shared by twice the frames.  4-byte complex samples and quadratic taps stay at 8 (16
-            // cost them 128 registers).  Measured on B200, chunks of 8 / 16: complex64 12 frames x 3
-            // transmits 299 / 236 us, 64 frames 339 / 301 us, 192 frames x 5 3.97 / 3.80 ms; FP16
-            // pairs, 192 frames 3.08 / 3.47 ms; complex64 quadratic, 12 frames 311 / 356 us.
-            const bool sixteen = esz == 8 && interp != kQuadratic && padded % 16 == 0;
-            const bool eight = cplx ? !sixteen : (!rows_ok && real8_ok);
-            p.lp.kind = eight ? kKindLaneVoxel8 : kKindLaneVoxel16;
-            p.lp.pad_frames = !rows_ok && !real8_ok ? static_cast<int>(padded) : 0;
-            p.lp.frame_chunks = static_cast<int>((eight && !cplx ? n_frames : padded) / (eight ? 8 : 16));
-        }
-        p.lp.passes = static_cast<int>(n_frames);
-        p.lp.block = dim3(kLaneVoxelThreads, 1, 1);
-        // One-frame jobs split each voxel's elements over 2 or 4 lanes.  Measured on B200: 4
-        // for jobs of fewer than 4 CTAs of 128 voxels per SM and for split delays, 2 otherwise.
-        int cs = 1;
-        if (n_frames <= 1) {
-            if (o.lanes_per_voxel == 1 || o.lanes_per_voxel == 2 || o.lanes_per_voxel == 4) {
-                cs = o.lanes_per_voxel;
-            } else {
-                const bool small = (n_vox + kLaneVoxelThreads - 1) / kLaneVoxelThreads < 4u * 148u;
-                cs = small || (o.flags & MACH_B200_FLAG_SPLIT_DELAY) ? 4 : 2;
-            }
-        }
-        p.lp.lanes_per_voxel = cs;
-        const int vpc = kLaneVoxelThreads / cs;  // voxels per CTA
-        const int chunk = o.tx_chunk > 0 ? o.tx_chunk
-                                         : cs * ((o.flags & MACH_B200_FLAG_SPLIT_DELAY) ? kMaxTxChunkSplit : kMaxTxChunk);
-        const uint32_t chunks = std::max<uint32_t>(1u, (n_tx + chunk - 1) / chunk);
-        p.lp.tx_chunk = static_cast<int>(std::max<uint32_t>(1u, (n_tx + chunks - 1) / chunks));
-        p.lp.grid = dim3(static_cast<unsigned>((n_vox + vpc - 1) / vpc), 1, 1);
-        // On a known grid: CTA tiles of wf x (128 / wf) voxels, warps of wf x (32 / wf).
-        // Automatic: 2 along the contiguous axis for 16 frames (rows of 32+ bytes), else 4.
-        const int wf = o.tile_fast == 1 || o.tile_fast == 2 || o.tile_fast == 4 || o.tile_fast == 8 ||
-                               o.tile_fast == 16
-                           ? o.tile_fast
-                           : (n_frames >= 16 ? 2 : 4);
-        if (grid_matches(o, n_vox) && o.grid_shape[2] >= wf) {
+        // One launch of `lanes` lanes per voxel over `chunks` frame chunks from frame `first`.
+        const bool split = (o.flags & MACH_B200_FLAG_SPLIT_DELAY) != 0u;
+        const bool wf_set = o.tile_fast == 1 || o.tile_fast == 2 || o.tile_fast == 4 || o.tile_fast == 8 || o.tile_fast == 16;
+        auto part = [&](int part_kind, int lanes, uint32_t first, uint32_t chunks, int wf_auto) {
+            LaunchPlan lp{};
+            lp.kind = part_kind;
+            lp.lanes_per_voxel = lanes;
+            lp.frame_first = static_cast<int>(first);
+            lp.frame_chunks = static_cast<int>(chunks);
+            lp.passes = static_cast<int>(n_frames);
+            lp.block = dim3(kLaneVoxelThreads, 1, 1);
+            const int vpc = kLaneVoxelThreads / lanes;  // voxels per CTA
+            const int cap = o.tx_chunk > 0 ? o.tx_chunk : lanes * (split ? kMaxTxChunkSplit : kMaxTxChunk);
+            const uint32_t tx_passes = std::max<uint32_t>(1u, (n_tx + cap - 1) / cap);
+            lp.tx_chunk = static_cast<int>(std::max<uint32_t>(1u, (n_tx + tx_passes - 1) / tx_passes));
+            lp.grid = dim3(static_cast<unsigned>((n_vox + vpc - 1) / vpc), 1, 1);
+            // On a known grid: CTA tiles of wf x (vpc / wf) voxels, warps of wf x (32 / lanes / wf).
+            const int wf = wf_set ? o.tile_fast : wf_auto;
             const int lw = wf == 1 ? 0 : (wf == 2 ? 1 : (wf == 4 ? 2 : (wf == 8 ? 3 : 4)));
-            p.lp.map_fast = o.grid_shape[2];
-            p.lp.map_wlog = lw;
             // Heaviest tiles first (measured on B200: compounding 1.90 -> 1.72 ms, Doppler
             // complex64 4.06 -> 3.84 ms, FP16 2.75 -> 2.48 ms; 3-D 16 frames 67.3 -> 67.8 ms,
-            // so 16-frame jobs keep the grid order).
-            p.lp.tile_rev = o.tile_order == 1 ? 1 : (o.tile_order == 2 ? 0 : (p.lp.kind == kKindLaneVoxel16 ? 0 : 1));
-            p.lp.map_outer = static_cast<int64_t>(n_vox / static_cast<uint64_t>(o.grid_shape[2]));
-            const int64_t per_outer = vpc >> lw;
-            const int64_t tiles = ((p.lp.map_outer + per_outer - 1) / per_outer) * ((p.lp.map_fast + wf - 1) / wf);
-            p.lp.grid = dim3(static_cast<unsigned>(tiles), 1, 1);
+            // so 16-frame jobs of real samples keep the grid order).
+            const int rev = o.tile_order == 1 ? 1 : (o.tile_order == 2 ? 0 : (part_kind == kKindLaneVoxel16 ? 0 : 1));
+            if (grid_matches(o, n_vox) && o.grid_shape[2] >= wf) {
+                lp.map_fast = o.grid_shape[2];
+                lp.map_wlog = lw;
+                lp.tile_rev = rev;
+                lp.map_outer = static_cast<int64_t>(n_vox / static_cast<uint64_t>(o.grid_shape[2]));
+                const int64_t per_outer = vpc >> lw;
+                const int64_t tiles = ((lp.map_outer + per_outer - 1) / per_outer) * ((lp.map_fast + wf - 1) / wf);
+                lp.grid = dim3(static_cast<unsigned>(tiles), 1, 1);
+            } else if (probe && n_frames > 8) {
+                lp.probe_grid = true;
+                lp.map_wlog = lw;
+                lp.tile_rev = rev;
+                lp.grid = dim3(static_cast<unsigned>(probed_tiles(static_cast<int64_t>(n_vox), vpc, wf)), 1, 1);
+            }
+            if (chunks > 1) lp.grid.x *= chunks;  // the chunks of a tile on consecutive CTAs
+            // split mode stages three words per (transmit, voxel): base, fraction, phase cycles
+            lp.smem = static_cast<size_t>(lp.tx_chunk) * vpc * sizeof(float) * (split ? 3 : 1);
+            return lp;
+        };
+        if (n_frames <= 1) {
+            // One-frame jobs split each voxel's elements over 2 or 4 lanes.  Measured on B200: 4
+            // for jobs of fewer than 4 CTAs of 128 voxels per SM and for split delays (128^3 voxels
+            // would take 20.7 ms instead of 21.4 ms with 2, but its longer sums double the rounding
+            // error, 4e-7 to 8e-7), 2 otherwise.
+            int cs = o.lanes_per_voxel;
+            if (cs != 1 && cs != 2 && cs != 4) {
+                cs = split || (n_vox + kLaneVoxelThreads - 1) / kLaneVoxelThreads < 4u * 148u ? 4 : 2;
+            }
+            p.lp = part(kKindLaneVoxel1, cs, 0, 0, 4);
+        } else if (n_frames <= 8) {
+            p.lp = part(kKindLaneVoxelN, 1, 0, 0, 4);
+        } else if (!cplx) {
+            // 2 voxels along the contiguous axis for rows of 32 bytes or more
+            const bool eight = !rows_ok && real8_ok;
+            p.lp = part(eight ? kKindLaneVoxel8 : kKindLaneVoxel16, 1, 0, eight ? n_frames / 8 : padded / 16,
+                        n_frames >= 16 ? 2 : 4);
+            p.lp.pad_frames = !rows_ok && !real8_ok ? static_cast<int>(padded) : 0;
+        } else {
+            // Groups of 4 lanes take 32 frames of a voxel, 2 lanes 16, and what is left runs in a second
+            // launch.  24 frames alone run as three chunks of the one-lane kernel (complex64 295 us
+            // against 309 us and 324 us with 2 and 4 lanes); 24 left over as one more, partly empty
+            // chunk of 4 lanes.  Warps lie across the contiguous axis for complex64 (fewest rows: 192
+            // frames 2.93 / 3.01 ms with 1 / 2 voxels along it), 4-byte pairs are within 2 %.
+            const uint32_t fours = padded / 32, rest = padded % 32;
+            const int wf4 = esz == 8 ? 1 : 4, wf2 = esz == 8 ? 1 : 2;
+            if (fours > 0) {
+                p.lp = part(kKindFrameGroup, 4, 0, fours + (rest == 24 ? 1 : 0), wf4);
+                if (rest == 8 || rest == 16) {
+                    p.rest = rest == 8 ? part(kKindLaneVoxel8, 1, fours * 32, 1, 2) : part(kKindFrameGroup, 2, fours * 32, 1, wf2);
+                    p.has_rest = true;
+                }
+            } else {
+                p.lp = padded == 16 ? part(kKindFrameGroup, 2, 0, 1, wf2) : part(kKindLaneVoxel8, 1, 0, padded / 8, 2);
+            }
+            p.lp.pad_frames = !rows_ok ? static_cast<int>(padded) : 0;
         }
-        else if (probe && n_frames > 8) {
-            p.lp.probe_grid = true;
-            p.lp.map_wlog = wf == 1 ? 0 : (wf == 2 ? 1 : (wf == 4 ? 2 : (wf == 8 ? 3 : 4)));
-            p.lp.tile_rev = p.lp.kind == kKindLaneVoxel16 ? 0 : 1;
-            p.lp.grid = dim3(static_cast<unsigned>(probed_tiles(static_cast<int64_t>(n_vox), vpc, wf)), 1, 1);
-        }
-        if (p.lp.frame_chunks > 1) p.lp.grid.x *= static_cast<unsigned>(p.lp.frame_chunks);  // consecutive CTAs
         // Element blocks: one launch per block of elements whose channel data (all transmits)
         // fits in L2 with room to spare.  Automatic for 16-frame jobs above 126 MB of channel
         // data (3-D: every CTA sweeps every (transmit, element) row set, and CTAs that drift apart
         // evict each other's rows; measured DRAM reads were 70x the channel data in one launch).
-        {
-            const uint64_t per_elem = static_cast<uint64_t>(n_tx) * n_samples * std::max<uint32_t>(n_frames, p.lp.pad_frames) * esz;
-            int eb = o.element_block;
-            if (eb == 0 && p.lp.kind == kKindLaneVoxel16 && per_elem > 0 &&
-                per_elem * n_rx > (uint64_t{126} << 20) && !batch) {
-                eb = static_cast<int>(std::max<uint64_t>(32, ((uint64_t{80} << 20) / per_elem) / 32 * 32));
-            }
-            p.lp.element_block = eb > 0 ? eb : 0;
+        const uint64_t per_elem = static_cast<uint64_t>(n_tx) * n_samples * std::max<uint32_t>(n_frames, p.lp.pad_frames) * esz;
+        int eb = o.element_block;
+        if (eb == 0 && (p.lp.kind == kKindLaneVoxel16 || n_frames == 16) && per_elem > 0 &&
+            per_elem * n_rx > (uint64_t{126} << 20) && !batch) {
+            eb = static_cast<int>(std::max<uint64_t>(32, ((uint64_t{80} << 20) / per_elem) / 32 * 32));
         }
-        // split mode stages three words per (transmit, voxel): base, fraction, phase cycles
-        p.lp.smem = static_cast<size_t>(p.lp.tx_chunk) * vpc * sizeof(float) *
-                    ((o.flags & MACH_B200_FLAG_SPLIT_DELAY) ? 3 : 1);
+        p.lp.element_block = eb > 0 ? eb : 0;
         return p;
     }
     if (kind == MACH_B200_KERNEL_STAGED) {
@@ -664,7 +683,31 @@ struct DeviceBuffer {
 bool lane_voxel_plan(const Plan& plan) {
     return !plan.staged && !plan.ensemble && !plan.frame_lane &&
            (plan.lp.kind == kKindLaneVoxel1 || plan.lp.kind == kKindLaneVoxelN || plan.lp.kind == kKindLaneVoxel16 ||
-            plan.lp.kind == kKindLaneVoxel8);
+            plan.lp.kind == kKindLaneVoxel8 || plan.lp.kind == kKindFrameGroup);
+}
+
+// Arguments that one launch of a plan sets.
+void apply_launch(DasArgs& a, const LaunchPlan& lp) {
+    a.frame_passes = lp.passes;
+    a.tx_chunk = lp.tx_chunk;
+    a.map_fast = lp.map_fast;
+    a.map_wlog = lp.map_wlog;
+    a.tile_rev = lp.tile_rev;
+    a.map_outer = lp.map_outer;
+    a.frame_chunks = lp.frame_chunks;
+    a.frame_first = lp.frame_first;
+}
+
+// The launches of a plan over the transmits and elements of `a`.
+cudaError_t dispatch_parts(int storage, const DasArgs& a, int interp, const Plan& plan, const CUtensorMap& map,
+                           cudaStream_t st) {
+    const cudaError_t e = dispatch(storage, a, interp, plan, map, st);
+    if (e != cudaSuccess || !plan.has_rest) return e;
+    DasArgs r = a;
+    apply_launch(r, plan.rest);
+    Plan second;
+    second.lp = plan.rest;
+    return dispatch(storage, r, interp, second, map, st);
 }
 
 // Whether a staging buffer of `bytes` leaves at least as much device memory free (else the
@@ -721,7 +764,7 @@ int dispatch_split(int storage, DasArgs a, int interp, const Plan& plan, cudaStr
             b.e_begin = e0;
             b.e_end = std::min(a.n_rx, e0 + eblk);
             b.accumulate = (t0 == 0 && e0 == 0) ? a.accumulate : 1;
-            MACH_B200_CUDA_TRY(dispatch(storage, b, interp, pl, map, st));
+            MACH_B200_CUDA_TRY(dispatch_parts(storage, b, interp, pl, map, st));
             e0 += eblk;
         } while (e0 < a.n_rx);
     }
@@ -899,13 +942,7 @@ int compound_impl(int32_t storage, const void* channel_data, const float* rx_coo
         plan = make_plan(false);
     }
     plan.st.status = dev->status;
-    a.frame_passes = plan.lp.passes;
-    a.tx_chunk = plan.lp.tx_chunk;
-    a.map_fast = plan.lp.map_fast;
-    a.map_wlog = plan.lp.map_wlog;
-    a.tile_rev = plan.lp.tile_rev;
-    a.map_outer = plan.lp.map_outer;
-    a.frame_chunks = plan.lp.frame_chunks;
+    apply_launch(a, plan.lp);
 
     if (all_device) {
         a.channel = channel_data;
@@ -1021,7 +1058,7 @@ int compound_impl(int32_t storage, const void* channel_data, const float* rx_coo
             b.accumulate = (k > 0 || !overwrite) ? 1 : 0;
             CUtensorMap map;
             std::memset(&map, 0, sizeof(map));
-            MACH_B200_CUDA_TRY(dispatch(storage, b, interp_type, plan, map, stream));
+            MACH_B200_CUDA_TRY(dispatch_parts(storage, b, interp_type, plan, map, stream));
         }
     } else {
         // Transmit chunks (>= 64 MB, at most 8 of them) copied on a side stream while the
@@ -1533,7 +1570,8 @@ int noalloc_impl(int32_t storage, const void* channel_data, const float* rx_coor
 struct mach_b200_batch {
     int device = 0;
     uint32_t max_jobs = 0;
-    static constexpr int kMaxGroups = 32;
+    static constexpr int kMaxGroups = 64;
+    static constexpr uint32_t kMaxParts = 2;  // launches of one job (Plan::rest)
     // pinned host tables (filled on the host, copied by the stream)
     BatchJob* h_jobs = nullptr;
     int64_t* h_begin = nullptr;
@@ -1550,10 +1588,10 @@ struct mach_b200_batch {
 namespace {
 
 struct GroupKey {
-    int family;  // 0 lane-voxel, 1 staged, 2 frame-lane
+    int family;  // 0 lane-voxel, 1 staged, 2 frame-lane, 3 frame-group
     int storage;
     int interp;
-    int variant;  // lane-voxel frame class (1, 0, 16) or staged lanes per voxel
+    int variant;  // lane-voxel frame class (1, 12, 14, 0, 8, 16) or staged / frame-group lanes per voxel
     int split;
     bool operator==(const GroupKey& o) const {
         return family == o.family && storage == o.storage && interp == o.interp && variant == o.variant &&
@@ -1566,6 +1604,7 @@ cudaError_t launch_group(const GroupKey& k, const PersistentLaunch& pl, cudaStre
     case S:                                                                                                   \
         return k.family == 0   ? launch_lane_voxel_persistent<S>(k.interp, k.variant, k.split != 0, pl, st)   \
                : k.family == 2 ? launch_frame_lane_persistent<S>(k.interp, k.variant, k.split != 0, pl, st)   \
+               : k.family == 3 ? launch_frame_group_persistent<S>(k.interp, k.variant, k.split != 0, pl, st)  \
                                : launch_staged_persistent<S>(k.interp, k.variant, pl, st);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     switch (k.storage) {
@@ -1579,6 +1618,7 @@ cudaError_t launch_group(const GroupKey& k, const PersistentLaunch& pl, cudaStre
         default:
             return k.family == 0   ? launch_lane_voxel_persistent<kCI16>(k.interp, k.variant, k.split != 0, pl, st)
                    : k.family == 2 ? launch_frame_lane_persistent<kCI16>(k.interp, k.variant, k.split != 0, pl, st)
+                   : k.family == 3 ? launch_frame_group_persistent<kCI16>(k.interp, k.variant, k.split != 0, pl, st)
                                    : launch_staged_persistent<kCI16>(k.interp, k.variant, pl, st);
     }
 #undef MACH_B200_GCASE
@@ -1607,13 +1647,13 @@ int batch_create(uint32_t max_jobs, mach_b200_batch** out) {
     if (max_jobs == 0 || max_jobs > (1u << 20)) return fail(MACH_B200_ERR_VALUE, "max_jobs must be in [1, 2^20]");
     auto* b = new mach_b200_batch();
     b->max_jobs = max_jobs;
-    const size_t G = mach_b200_batch::kMaxGroups;
+    const size_t G = mach_b200_batch::kMaxGroups, P = mach_b200_batch::kMaxParts;
     cudaError_t e = cudaGetDevice(&b->device);
-    if (e == cudaSuccess) e = cudaMallocHost(&b->h_jobs, sizeof(BatchJob) * max_jobs);
-    if (e == cudaSuccess) e = cudaMallocHost(&b->h_begin, sizeof(int64_t) * max_jobs);
+    if (e == cudaSuccess) e = cudaMallocHost(&b->h_jobs, sizeof(BatchJob) * max_jobs * P);
+    if (e == cudaSuccess) e = cudaMallocHost(&b->h_begin, sizeof(int64_t) * max_jobs * P);
     if (e == cudaSuccess) e = cudaMallocHost(&b->h_hdr, sizeof(BatchHeader) * G);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_jobs, sizeof(BatchJob) * max_jobs);
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_begin, sizeof(int64_t) * max_jobs);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_jobs, sizeof(BatchJob) * max_jobs * P);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_begin, sizeof(int64_t) * max_jobs * P);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_hdr, sizeof(BatchHeader) * G);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counters, sizeof(unsigned long long) * G);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->copied, cudaEventDisableTiming);
@@ -1646,8 +1686,14 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
     // ---- plan every job, assign it to a group (kernel signature)
     GroupKey keys[mach_b200_batch::kMaxGroups];
     int n_groups = 0;
-    std::vector<int> group_of(n_jobs), order;
     std::vector<Plan> plans(n_jobs);
+    struct Part {  // one launch of one job
+        uint32_t job;
+        const LaunchPlan* lp;
+        int group;
+    };
+    std::vector<Part> parts;
+    parts.reserve(mach_b200_batch::kMaxParts * static_cast<size_t>(n_jobs));
     for (uint32_t i = 0; i < n_jobs; ++i) {
         const mach_b200_job& j = jobs[i];
         if ((rc = check_args(j.storage, j.interp_type, j.tukey_alpha, j.n_tx, j.n_rx, j.n_samples, j.n_scan,
@@ -1671,41 +1717,45 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         o.lanes_per_voxel = j.lanes_per_voxel;
         plans[i] = plan_launch(j.storage, j.n_scan, j.n_frames, j.n_tx, j.channel_data, true, o, j.interp_type, true);
         const Plan& p = plans[i];
-        GroupKey k{};
-        if (p.frame_lane) {
-            k = {2, j.storage, j.interp_type, p.lp.frame_slots, (j.flags & MACH_B200_FLAG_SPLIT_DELAY) ? 1 : 0};
-        } else if (p.staged) {
-            k = {1, j.storage, j.interp_type, p.lp.lanes_per_voxel, 0};
-        } else if (p.lp.kind == kKindLaneVoxel1 || p.lp.kind == kKindLaneVoxelN || p.lp.kind == kKindLaneVoxel16 ||
-                   p.lp.kind == kKindLaneVoxel8) {
-            int fc = p.lp.kind == kKindLaneVoxel1 ? 1
-                     : (p.lp.kind == kKindLaneVoxel16 ? 16 : (p.lp.kind == kKindLaneVoxel8 ? 8 : 0));
-            if (fc == 1 && p.lp.lanes_per_voxel > 1) fc = 10 + p.lp.lanes_per_voxel;  // 12 / 14
-            k = {0, j.storage, j.interp_type, fc, (j.flags & MACH_B200_FLAG_SPLIT_DELAY) ? 1 : 0};
-        } else {
-            return fail(MACH_B200_ERR_VALUE, "job %u: %u frames not a multiple of the storage's lane vector", i,
-                        j.n_frames);
+        for (const LaunchPlan* lp : {&p.lp, p.has_rest ? &p.rest : nullptr}) {
+            if (!lp) continue;
+            GroupKey k{};
+            const int split = (j.flags & MACH_B200_FLAG_SPLIT_DELAY) ? 1 : 0;
+            if (p.frame_lane) {
+                k = {2, j.storage, j.interp_type, lp->frame_slots, split};
+            } else if (p.staged) {
+                k = {1, j.storage, j.interp_type, lp->lanes_per_voxel, 0};
+            } else if (lp->kind == kKindFrameGroup) {
+                k = {3, j.storage, j.interp_type, lp->lanes_per_voxel, split};
+            } else if (lp->kind == kKindLaneVoxel1) {
+                k = {0, j.storage, j.interp_type, lp->lanes_per_voxel > 1 ? 10 + lp->lanes_per_voxel : 1, split};
+            } else if (lp->kind == kKindLaneVoxelN || lp->kind == kKindLaneVoxel16 || lp->kind == kKindLaneVoxel8) {
+                k = {0, j.storage, j.interp_type, lp->kind == kKindLaneVoxel16 ? 16 : (lp->kind == kKindLaneVoxel8 ? 8 : 0), split};
+            } else {
+                return fail(MACH_B200_ERR_VALUE, "job %u: %u frames not a multiple of the storage's lane vector", i,
+                            j.n_frames);
+            }
+            int gi = 0;
+            while (gi < n_groups && !(keys[gi] == k)) ++gi;
+            if (gi == n_groups) {
+                if (n_groups == mach_b200_batch::kMaxGroups) return fail(MACH_B200_ERR_VALUE, "too many kernel signatures");
+                keys[n_groups++] = k;
+            }
+            parts.push_back({i, lp, gi});
         }
-        int gi = 0;
-        while (gi < n_groups && !(keys[gi] == k)) ++gi;
-        if (gi == n_groups) {
-            if (n_groups == mach_b200_batch::kMaxGroups) return fail(MACH_B200_ERR_VALUE, "too many kernel signatures");
-            keys[n_groups++] = k;
-        }
-        group_of[i] = gi;
     }
 
     // ---- fill the pinned tables, grouped
     std::vector<int> first(n_groups + 1, 0);
-    for (uint32_t i = 0; i < n_jobs; ++i) ++first[group_of[i] + 1];
+    for (const Part& part : parts) ++first[part.group + 1];
     for (int g = 0; g < n_groups; ++g) first[g + 1] += first[g];
     std::vector<int> fill(first.begin(), first.end() - 1);
     std::vector<size_t> smem(n_groups, 0);
     std::vector<int64_t> items(n_groups, 0);
     std::vector<int> max_items(n_groups, 0);
-    for (uint32_t i = 0; i < n_jobs; ++i) {
-        const mach_b200_job& j = jobs[i];
-        const int g = group_of[i];
+    for (const Part& part : parts) {
+        const mach_b200_job& j = jobs[part.job];
+        const int g = part.group;
         const int slot = fill[g]++;
         BatchJob& bj = b->h_jobs[slot];
         std::memset(&bj, 0, sizeof(bj));
@@ -1719,21 +1769,15 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         bj.a.out = j.out;
         bj.a.n_tx = static_cast<int32_t>(need_channel ? j.n_tx : 0);
         bj.a.accumulate = (j.flags & MACH_B200_FLAG_OVERWRITE) ? 0 : 1;
-        const Plan& p = plans[i];
-        bj.a.frame_passes = p.lp.passes;
-        bj.a.tx_chunk = p.lp.tx_chunk;
-        bj.a.map_fast = p.lp.map_fast;
-        bj.a.map_wlog = p.lp.map_wlog;
-        bj.a.tile_rev = p.lp.tile_rev;
-        bj.a.map_outer = p.lp.map_outer;
-        bj.a.frame_chunks = p.lp.frame_chunks;
+        const Plan& p = plans[part.job];
+        apply_launch(bj.a, *part.lp);
         bj.st = p.st;
         bj.st.status = dev->status;
         bj.fl = p.fl;
-        bj.tiles = static_cast<int32_t>(p.lp.grid.x);
-        bj.chunks = static_cast<int32_t>(p.staged ? p.lp.grid.y : 1);
+        bj.tiles = static_cast<int32_t>(part.lp->grid.x);
+        bj.chunks = static_cast<int32_t>(p.staged ? part.lp->grid.y : 1);
         if (p.staged && p.st.use_tma && bj.a.n_tx > 0) {
-            const int fc = p.lp.lanes_per_voxel * static_cast<int>(8 / storage_bytes(j.storage));
+            const int fc = part.lp->lanes_per_voxel * static_cast<int>(8 / storage_bytes(j.storage));
             if ((rc = encode_channel_map(&bj.map, j.storage, j.channel_data,
                                          static_cast<uint64_t>(j.n_tx) * j.n_rx * j.n_samples, j.n_frames, fc,
                                          p.st.window_rows))) {
@@ -1743,7 +1787,7 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         const int64_t job_items = static_cast<int64_t>(bj.tiles) * bj.chunks;
         b->h_begin[slot] = items[g];
         items[g] += job_items;
-        smem[g] = std::max(smem[g], p.lp.smem);
+        smem[g] = std::max(smem[g], part.lp->smem);
     }
     for (int g = 0; g < n_groups; ++g) {
         b->h_hdr[g].n_items = items[g];
@@ -1753,8 +1797,8 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
 
     // ---- copies, counters, one persistent launch per group
     if (n_jobs) {
-        MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_jobs, b->h_jobs, sizeof(BatchJob) * n_jobs, cudaMemcpyHostToDevice, stream));
-        MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_begin, b->h_begin, sizeof(int64_t) * n_jobs, cudaMemcpyHostToDevice, stream));
+        MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_jobs, b->h_jobs, sizeof(BatchJob) * parts.size(), cudaMemcpyHostToDevice, stream));
+        MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_begin, b->h_begin, sizeof(int64_t) * parts.size(), cudaMemcpyHostToDevice, stream));
         MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_hdr, b->h_hdr, sizeof(BatchHeader) * n_groups, cudaMemcpyHostToDevice, stream));
         MACH_B200_CUDA_TRY(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned long long) * n_groups, stream));
         // While capturing a graph the copies run at replay time, from the tables as they are then.
