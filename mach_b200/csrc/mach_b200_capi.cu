@@ -1583,6 +1583,12 @@ struct mach_b200_batch {
     unsigned long long* d_counters = nullptr;
     cudaEvent_t copied = nullptr;  // host tables may be rewritten once this has passed
     bool pending = false;
+    // The launches of one run are independent: they go to the caller's stream and these, forked
+    // from it and joined to it again, so that one launch's last tiles run beside the next one's
+    // first (five launches of a mixed batch on B200: 744 us one after the other, 623 us so).
+    static constexpr int kSideStreams = 3;
+    cudaStream_t side[kSideStreams] = {};
+    cudaEvent_t forked = nullptr, joined[kSideStreams] = {};
 };
 
 namespace {
@@ -1630,6 +1636,11 @@ void batch_free(mach_b200_batch* b) {
         cudaEventSynchronize(b->copied);
         cudaEventDestroy(b->copied);
     }
+    for (int i = 0; i < mach_b200_batch::kSideStreams; ++i) {
+        if (b->side[i]) cudaStreamDestroy(b->side[i]);
+        if (b->joined[i]) cudaEventDestroy(b->joined[i]);
+    }
+    if (b->forked) cudaEventDestroy(b->forked);
     cudaFreeHost(b->h_jobs);
     cudaFreeHost(b->h_begin);
     cudaFreeHost(b->h_hdr);
@@ -1657,6 +1668,11 @@ int batch_create(uint32_t max_jobs, mach_b200_batch** out) {
     if (e == cudaSuccess) e = cudaMalloc(&b->d_hdr, sizeof(BatchHeader) * G);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counters, sizeof(unsigned long long) * G);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->copied, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming);
+    for (int i = 0; i < mach_b200_batch::kSideStreams; ++i) {
+        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->joined[i], cudaEventDisableTiming);
+    }
     if (e != cudaSuccess) {
         batch_free(b);
         return fail(MACH_B200_ERR_CUDA, "batch context allocation failed: %s", cudaGetErrorString(e));
@@ -1753,6 +1769,7 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
     std::vector<size_t> smem(n_groups, 0);
     std::vector<int64_t> items(n_groups, 0);
     std::vector<int> max_items(n_groups, 0);
+    std::vector<double> points(n_groups, 0.0);
     for (const Part& part : parts) {
         const mach_b200_job& j = jobs[part.job];
         const int g = part.group;
@@ -1787,6 +1804,7 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         const int64_t job_items = static_cast<int64_t>(bj.tiles) * bj.chunks;
         b->h_begin[slot] = items[g];
         items[g] += job_items;
+        points[g] += static_cast<double>(j.n_scan) * j.n_rx * j.n_tx * j.n_frames;
         smem[g] = std::max(smem[g], part.lp->smem);
     }
     for (int g = 0; g < n_groups; ++g) {
@@ -1810,13 +1828,27 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         }
     }
     bool any_waits = false;  // staged kernels have bounded waits
+    std::vector<int> order;  // the groups with work, most points first
     for (int g = 0; g < n_groups; ++g) {
-        if (items[g] == 0) continue;
+        if (items[g] > 0) order.push_back(g);
+    }
+    std::sort(order.begin(), order.end(), [&](int x, int y) { return points[x] > points[y]; });
+    const int n_side = std::min<int>(mach_b200_batch::kSideStreams, static_cast<int>(order.size()) - 1);
+    if (n_side > 0) MACH_B200_CUDA_TRY(cudaEventRecord(b->forked, stream));
+    for (int i = 0; i < n_side; ++i) MACH_B200_CUDA_TRY(cudaStreamWaitEvent(b->side[i], b->forked, 0));
+    cudaError_t launched = cudaSuccess;
+    for (size_t k = 0; k < order.size() && launched == cudaSuccess; ++k) {
+        const int g = order[k], lane = static_cast<int>(k) % (n_side + 1);
         PersistentLaunch pl{b->d_hdr + g, b->d_jobs + first[g], b->d_begin + first[g], b->d_counters + g, smem[g],
                             max_items[g]};
         any_waits |= keys[g].family == 1;
-        MACH_B200_CUDA_TRY(launch_group(keys[g], pl, stream));
+        launched = launch_group(keys[g], pl, lane == 0 ? stream : b->side[lane - 1]);
     }
+    for (int i = 0; i < n_side; ++i) {  // joined also after a failed launch
+        MACH_B200_CUDA_TRY(cudaEventRecord(b->joined[i], b->side[i]));
+        MACH_B200_CUDA_TRY(cudaStreamWaitEvent(stream, b->joined[i], 0));
+    }
+    MACH_B200_CUDA_TRY(launched);
     if (!(flags & MACH_B200_FLAG_ASYNC)) {
         MACH_B200_CUDA_TRY(cudaStreamSynchronize(stream));
         b->pending = false;
