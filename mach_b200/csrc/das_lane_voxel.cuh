@@ -1080,11 +1080,15 @@ __device__ __forceinline__ float2 gather_taps(const typename Storage<S>::T* row,
 
 // CTAs per SM that the register budget is cut for, from the state a point keeps live: 16 frames of
 // 16-bit real samples fit 72 registers, of float32 96; 8 complex64 frames 72 (quadratic: three
-// rows in flight, 96); the other kernels 64.
+// rows in flight, 96).  One real frame runs in 40 (the loads of one volume of int16 wait less with more
+// warps: 8 / 12 / 16 CTAs 21.4 / 20.1 / 20.2 ms with split delays, 18.5 / 17.2 / 18.7 ms with FP32
+// delays), one complex frame in up to 72 (75 transmits of complex64 7 / 8 / 10 CTAs 1.43 / 1.44 / 1.62 ms,
+// 11 of FP16 pairs 159 / 166 / 177 us); the other kernels 64.
 template <int S, int INTERP, int NF>
 constexpr int lane_voxel_ctas() {
     if (NF == 16) return S == kF32 ? 5 : 7;
     if (NF == 8 && S == kC64) return INTERP == kQuadratic ? 5 : 7;
+    if (NF == 1) return Storage<S>::kComplex ? 7 : 12;
     return 8;
 }
 
