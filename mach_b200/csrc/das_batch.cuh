@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(kLaneVoxelThreads, lane_voxel_ctas<S, INTERP, 
 // (the arguments are read from shared memory here: one or two CTAs of registers more than the
 // per-job kernel)
 template <int S, int INTERP, int LF, bool SPLIT>
-__global__ void __launch_bounds__(kLaneVoxelThreads, frame_group_ctas<S, INTERP, LF>() - (LF == 4 ? 2 : 1))
+__global__ void __launch_bounds__(kLaneVoxelThreads, frame_group_ctas<S, INTERP, LF>() - (LF >= 4 ? 2 : 1))
     das_frame_group_persistent(const BatchHeader* __restrict__ hdr, const BatchJob* __restrict__ jobs,
                                const int64_t* __restrict__ item_begin, unsigned long long* counter) {
     extern __shared__ float smem_words[];

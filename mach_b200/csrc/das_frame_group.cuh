@@ -1,23 +1,22 @@
-// Frame-group gather kernel for complex ensembles: LF neighbouring lanes own one voxel, eight frames
-// each, and share the arithmetic of its delays.
+// Frame-group gather kernel for complex ensembles: LF = 2, 4, 8 or 16 neighbouring lanes own one voxel,
+// eight frames each, and share the arithmetic of its delays.
 //
 // A warp-wide 256-bit load of the voxel-per-lane kernel touched as many 128-byte lines as its 32
 // voxels had sample rows (about 16), and used 32 bytes of each: the L1 tag stage, not its data path,
 // bounded the kernel (200-frame complex64 Doppler: data pipe 72 %, time unchanged with twice the
 // loads in flight).  Here the lanes of a voxel read adjacent 32-byte pieces of one row, so a
-// load touches half or a quarter of the lines.  The delay arithmetic is not repeated by the
+// load touches fewer lines, and whole ones.  The delay arithmetic is not repeated by the
 // lanes of a voxel: each takes one of LF consecutive elements, forms the receive path and then, per
 // transmit, the tap row and weights of its own element; the LF points are then summed one after
 // the other by all of the voxel's lanes, their four parameters broadcast by warp shuffles.
 //
 // Measured on B200, 8-frame chunks of the voxel-per-lane kernel -> 4 lanes per voxel, 192 frames x 5
 // transmits on 256 x 256: complex64 3.80 -> 2.80 ms (nearest 2.87 -> 1.54, quadratic 5.70 -> 3.80),
-// FP16 pairs 3.08 -> 2.07 ms, int16 pairs 3.39 -> 2.74 ms; 16 frames x 3 with 2 lanes: complex64 223 ->
-// 193 us, FP16 pairs 208 -> 174 us.  Its loads now use whole lines (11 of at least 8 wavefronts per
-// request); it waits for them (complex64: issue 0.46 per cycle, 24-32 warps per SM), or for
-// issue (FP16 pairs: 0.73).  Rows that are no multiple of 128 bytes (200 frames: 1600 bytes) make a
-// voxel's piece straddle two lines: 200 frames x 5 took 3.60 -> 3.22 ms (complex64) and 2.80 -> 2.46 ms
-// (FP16 pairs).
+// FP16 pairs 3.08 -> 2.07 ms, int16 pairs 3.39 -> 2.74 ms; 8 lanes 2.56 ms (complex64) and 1.96 ms
+// (FP16 pairs); 128 frames with 4 / 8 / 16 lanes 1.84 / 1.70 / 1.57 ms and 1.39 / 1.31 / 1.26 ms; 16 frames
+// x 3 with 2 lanes: complex64 223 -> 193 us, FP16 pairs 208 -> 174 us.  What is left is load latency
+// (complex64 with 4 lanes: issue 0.46 per cycle) and issue (FP16 pairs: 0.73); rows that are no
+// multiple of 128 bytes (200 frames) make a voxel's piece straddle one line more.
 #pragma once
 
 #include "das_lane_voxel.cuh"
@@ -268,7 +267,7 @@ __device__ __forceinline__ void frame_group_tile(const DasArgs& a, int64_t tile,
 template <int S, int INTERP, int LF>
 constexpr int frame_group_ctas() {
     if (INTERP == kQuadratic) return S == kC64 ? 5 : 8;
-    if (LF == 4) return S == kC64 ? 8 : 10;
+    if (LF >= 4) return S == kC64 ? 8 : 10;
     return S == kC64 ? 6 : 8;
 }
 

@@ -23,13 +23,13 @@ enum KernelKind : int {
     kKindEnsemble = 6,     // das_ensemble_kernel, windows in tensor memory, lanes = frames
     kKindLaneVoxel8 = 7,   // das_lane_voxel_kernel, chunks of 8 frames (grid.y) of a longer ensemble
     kKindFrameLane = 8,    // das_frame_lane_kernel, lanes = frames, rows reused along voxel runs
-    kKindFrameGroup = 9,   // das_frame_group_kernel, 2 or 4 lanes per voxel, 8 complex frames each
+    kKindFrameGroup = 9,   // das_frame_group_kernel, 2 to 16 lanes per voxel, 8 complex frames each
 };
 
 struct LaunchPlan {
     int kind;
     int lanes_per_voxel;  // staged kernel: 4, 8, 16 or 32; one-frame lane-voxel kernel: 1, 2 or 4 lanes per voxel;
-                          // frame-group kernel: 2 or 4
+                          // frame-group kernel: 2, 4, 8 or 16
     int passes;       // frames per lane (multi-frame kernels)
     int tx_chunk;     // arrivals staged per pass (lane-voxel kernels)
     dim3 grid;
@@ -126,8 +126,12 @@ cudaError_t launch_das(const DasArgs& a, int interp, const LaunchPlan& p, cudaSt
         case kKindLaneVoxel8: MACH_B200_LV(I, 8); break;     \
         case kKindFrameGroup:                                \
             if constexpr (Storage<S>::kComplex) {            \
-                if (p.lanes_per_voxel == 4) MACH_B200_FG(I, 4); \
-                else MACH_B200_FG(I, 2);                     \
+                switch (p.lanes_per_voxel) {                 \
+                    case 16: MACH_B200_FG(I, 16); break;     \
+                    case 8: MACH_B200_FG(I, 8); break;       \
+                    case 4: MACH_B200_FG(I, 4); break;       \
+                    default: MACH_B200_FG(I, 2); break;      \
+                }                                            \
             }                                                \
             break;                                           \
         case kKindWarpHalf: MACH_B200_WG(I, 16, 4); break;   \
@@ -225,7 +229,7 @@ cudaError_t launch_lane_voxel_persistent(int interp, int frame_class, bool split
 #undef MACH_B200_PLV
 }
 
-// Frame-group family: variant = lanes per voxel (2, 4); complex storage.
+// Frame-group family: variant = lanes per voxel (2, 4, 8, 16); complex storage.
 template <int S>
 cudaError_t launch_frame_group_persistent(int interp, int lanes, bool split, const PersistentLaunch& pl,
                                           cudaStream_t stream) {
@@ -234,6 +238,8 @@ cudaError_t launch_frame_group_persistent(int interp, int lanes, bool split, con
     return split ? launch_persistent(das_frame_group_persistent<S, I, LF, true>, kLaneVoxelThreads, pl, stream) \
                  : launch_persistent(das_frame_group_persistent<S, I, LF, false>, kLaneVoxelThreads, pl, stream)
 #define MACH_B200_PFG_LF(I)          \
+    if (lanes == 16) MACH_B200_PFG(I, 16); \
+    if (lanes == 8) MACH_B200_PFG(I, 8); \
     if (lanes == 4) MACH_B200_PFG(I, 4); \
     MACH_B200_PFG(I, 2)
         switch (interp) {

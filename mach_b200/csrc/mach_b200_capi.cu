@@ -208,10 +208,12 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 constexpr int kMaxTxChunk = 40;
 constexpr int kMaxTxChunkSplit = 32;
 
+constexpr int kMaxRest = 3;
+
 struct Plan {
     LaunchPlan lp{};
-    LaunchPlan rest{};      // second launch of the frames that lp leaves (lane-voxel family)
-    bool has_rest = false;
+    LaunchPlan rest[kMaxRest] = {};  // further launches of the frames that lp leaves (lane-voxel family)
+    int n_rest = 0;
     StagedArgs st{};
     EnsembleArgs ea{};
     FrameLaneArgs fl{};
@@ -500,22 +502,34 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
                         n_frames >= 16 ? 2 : 4);
             p.lp.pad_frames = !rows_ok && !real8_ok ? static_cast<int>(padded) : 0;
         } else {
-            // Groups of 4 lanes take 32 frames of a voxel, 2 lanes 16, and what is left runs in a second
-            // launch.  24 frames alone run as three chunks of the one-lane kernel (complex64 295 us
-            // against 309 us and 324 us with 2 and 4 lanes); 24 left over as one more, partly empty
-            // chunk of 4 lanes.  Warps lie across the contiguous axis for complex64 (fewest rows: 192
-            // frames 2.93 / 3.01 ms with 1 / 2 voxels along it), 4-byte pairs are within 2 %.
-            const uint32_t fours = padded / 32, rest = padded % 32;
-            const int wf4 = esz == 8 ? 1 : 4, wf2 = esz == 8 ? 1 : 2;
-            if (fours > 0) {
-                p.lp = part(kKindFrameGroup, 4, 0, fours + (rest == 24 ? 1 : 0), wf4);
-                if (rest == 8 || rest == 16) {
-                    p.rest = rest == 8 ? part(kKindLaneVoxel8, 1, fours * 32, 1, 2) : part(kKindFrameGroup, 2, fours * 32, 1, wf2);
-                    p.has_rest = true;
-                }
+            // Groups of 16, 8, 4 and 2 lanes take 128, 64, 32 and 16 frames of a voxel; the more, the
+            // cheaper a frame (das_frame_group.cuh), so the frames go to the widest group first, with
+            // a partly empty chunk where at least three quarters of it are used, and the last 8 to the
+            // one-lane kernel.  24 frames alone run as three chunks of that kernel (complex64 295 us
+            // against 309 us and 324 us with 2 and 4 lanes).  Warps lie across the contiguous axis for
+            // complex64 (fewest rows: 192 frames with 4 lanes 2.93 / 3.01 ms with 1 / 2 voxels along
+            // it); 4-byte pairs are within 2 %.
+            int n = 0;
+            LaunchPlan parts[kMaxRest + 1];
+            uint32_t at = 0, left = padded;
+            auto add = [&](int lanes, uint32_t chunks) {
+                if (chunks == 0) return;
+                parts[n++] = lanes == 1 ? part(kKindLaneVoxel8, 1, at, chunks, 2)
+                                        : part(kKindFrameGroup, lanes, at, chunks, esz == 8 ? 1 : (lanes == 4 ? 4 : 2));
+                at += 8u * lanes * chunks;
+                left = padded > at ? padded - at : 0;
+            };
+            if (padded == 24) {
+                add(1, 3);
             } else {
-                p.lp = padded == 16 ? part(kKindFrameGroup, 2, 0, 1, wf2) : part(kKindLaneVoxel8, 1, 0, padded / 8, 2);
+                add(16, (left + 31) / 128);
+                add(8, (left + 15) / 64);
+                add(4, (left + 8) / 32);
+                add(2, left / 16);
+                add(1, left / 8);
             }
+            p.lp = parts[0];
+            for (int k = 1; k < n; ++k) p.rest[p.n_rest++] = parts[k];
             p.lp.pad_frames = !rows_ok ? static_cast<int>(padded) : 0;
         }
         // Element blocks: one launch per block of elements whose channel data (all transmits)
@@ -701,13 +715,15 @@ void apply_launch(DasArgs& a, const LaunchPlan& lp) {
 // The launches of a plan over the transmits and elements of `a`.
 cudaError_t dispatch_parts(int storage, const DasArgs& a, int interp, const Plan& plan, const CUtensorMap& map,
                            cudaStream_t st) {
-    const cudaError_t e = dispatch(storage, a, interp, plan, map, st);
-    if (e != cudaSuccess || !plan.has_rest) return e;
-    DasArgs r = a;
-    apply_launch(r, plan.rest);
-    Plan second;
-    second.lp = plan.rest;
-    return dispatch(storage, r, interp, second, map, st);
+    cudaError_t e = dispatch(storage, a, interp, plan, map, st);
+    for (int k = 0; k < plan.n_rest && e == cudaSuccess; ++k) {
+        DasArgs r = a;
+        apply_launch(r, plan.rest[k]);
+        Plan further;
+        further.lp = plan.rest[k];
+        e = dispatch(storage, r, interp, further, map, st);
+    }
+    return e;
 }
 
 // Whether a staging buffer of `bytes` leaves at least as much device memory free (else the
@@ -1571,7 +1587,7 @@ struct mach_b200_batch {
     int device = 0;
     uint32_t max_jobs = 0;
     static constexpr int kMaxGroups = 64;
-    static constexpr uint32_t kMaxParts = 2;  // launches of one job (Plan::rest)
+    static constexpr uint32_t kMaxParts = 1 + kMaxRest;  // launches of one job
     // pinned host tables (filled on the host, copied by the stream)
     BatchJob* h_jobs = nullptr;
     int64_t* h_begin = nullptr;
@@ -1733,8 +1749,8 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         o.lanes_per_voxel = j.lanes_per_voxel;
         plans[i] = plan_launch(j.storage, j.n_scan, j.n_frames, j.n_tx, j.channel_data, true, o, j.interp_type, true);
         const Plan& p = plans[i];
-        for (const LaunchPlan* lp : {&p.lp, p.has_rest ? &p.rest : nullptr}) {
-            if (!lp) continue;
+        for (int part = 0; part <= p.n_rest; ++part) {
+            const LaunchPlan* lp = part == 0 ? &p.lp : &p.rest[part - 1];
             GroupKey k{};
             const int split = (j.flags & MACH_B200_FLAG_SPLIT_DELAY) ? 1 : 0;
             if (p.frame_lane) {

@@ -1,4 +1,4 @@
-"""Complex ensembles on groups of 2 and 4 lanes per voxel: every split of the frames into launches,
+"""Complex ensembles on groups of 2, 4, 8 and 16 lanes per voxel: every split of the frames into launches,
 every storage and interpolation, rows that end inside the image, small grids, and batches."""
 
 from __future__ import annotations
@@ -16,7 +16,7 @@ COMPLEX = ["c64", "cf16", "cbf16", "ci16"]
 
 @pytest.mark.parametrize("storage", COMPLEX)
 @pytest.mark.parametrize("interp", [0, 1, 2])
-@pytest.mark.parametrize("n_frames", [16, 24, 32, 40, 48, 56, 72])
+@pytest.mark.parametrize("n_frames", [16, 24, 32, 40, 48, 56, 72, 88, 104, 128, 168, 200])
 def test_matches_the_warp_kernel_and_oracle(cuda, storage, interp, n_frames):
     w = _workload(storage, n_frames, interp)
     got, warp = H.gpu_compound(w), H.gpu_compound(w, kernel="warp")
@@ -26,7 +26,7 @@ def test_matches_the_warp_kernel_and_oracle(cuda, storage, interp, n_frames):
 
 @pytest.mark.parametrize("delay", ["reference", "split"])
 @pytest.mark.parametrize("interp", [0, 1, 2])
-@pytest.mark.parametrize("n_frames,n_tx", [(16, 1), (40, 2), (64, 5)])
+@pytest.mark.parametrize("n_frames,n_tx", [(16, 1), (40, 2), (64, 5), (136, 2)])
 def test_rows_that_end_inside_the_image(cuda, delay, interp, n_frames, n_tx):
     w = H.small("doppler", n_frames=n_frames, n_tx=n_tx, n_samples=500)
     w.params["interp_type"] = interp
@@ -36,7 +36,7 @@ def test_rows_that_end_inside_the_image(cuda, delay, interp, n_frames, n_tx):
 
 
 @pytest.mark.parametrize("n_x,n_z", [(1, 1), (3, 5), (9, 33), (130, 7)])
-@pytest.mark.parametrize("n_frames", [16, 32, 40])
+@pytest.mark.parametrize("n_frames", [16, 32, 40, 64, 128])
 def test_tiling_never_changes_a_sum(cuda, n_x, n_z, n_frames):
     w = H.small("doppler", n_x=n_x, n_z=n_z, n_frames=n_frames, n_elements=40)
     base = H.gpu_compound(w, grid_shape=False)
@@ -44,7 +44,7 @@ def test_tiling_never_changes_a_sum(cuda, n_x, n_z, n_frames):
         np.testing.assert_array_equal(base, H.gpu_compound(w, **kw))
 
 
-@pytest.mark.parametrize("n_frames", [16, 32, 40, 48])
+@pytest.mark.parametrize("n_frames", [16, 32, 40, 48, 72, 128])
 @pytest.mark.parametrize("storage", ["c64", "cf16"])
 def test_batch_is_bit_identical(cuda, n_frames, storage):
     import torch
