@@ -458,7 +458,8 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
             lp.tx_chunk = static_cast<int>(std::max<uint32_t>(1u, (n_tx + tx_passes - 1) / tx_passes));
             lp.grid = dim3(static_cast<unsigned>((n_vox + vpc - 1) / vpc), 1, 1);
             // On a known grid: CTA tiles of wf x (vpc / wf) voxels, warps of wf x (32 / lanes / wf).
-            const int wf = wf_set ? o.tile_fast : wf_auto;
+            // (at most the CTA's voxels: 8 with 16 lanes per voxel)
+            const int wf = std::min(vpc, wf_set ? o.tile_fast : wf_auto);
             const int lw = wf == 1 ? 0 : (wf == 2 ? 1 : (wf == 4 ? 2 : (wf == 8 ? 3 : 4)));
             // Heaviest tiles first (measured on B200: compounding 1.90 -> 1.72 ms, Doppler
             // complex64 4.06 -> 3.84 ms, FP16 2.75 -> 2.48 ms; 3-D 16 frames 67.3 -> 67.8 ms,
