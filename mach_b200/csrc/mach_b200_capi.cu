@@ -1237,37 +1237,52 @@ int power_impl(int32_t storage, const void* channel_data, const float* rx_coords
     const size_t power_bytes = static_cast<size_t>(n_scan) * sizeof(float);
 
     // ---- fused: the ensemble / frame-lane kernel adds |x|^2 of each frame block into out
-    if (all_device && need_channel) {
-        Plan plan = plan_launch(storage, n_scan, n_frames, n_tx, channel_data, true, opt, interp_type, false, n_rx,
+    auto run_fused = [&](const mach_b200_options& options, bool* fused) -> int {
+        *fused = false;
+        if (!all_device || !need_channel) return MACH_B200_OK;
+        Plan plan = plan_launch(storage, n_scan, n_frames, n_tx, channel_data, true, options, interp_type, false, n_rx,
                                 n_samples, true);
         const int64_t per_tx = static_cast<int64_t>(n_rx) * n_samples * n_frames;
-        if ((plan.ensemble || plan.frame_lane) && per_tx * n_tx < (int64_t{1} << 31)) {
-            plan.st.status = dev->status;
-            DasArgs a = make_args(rx_coords_m, scan_coords_m, n_scan, n_rx, n_samples, n_frames, f_number, rx_start_s,
-                                  sampling_freq_hz, sound_speed_m_s, modulation_freq_hz, tukey_alpha, channel_scale,
-                                  cplx, flags);
-            a.frame_passes = plan.lp.passes;
-            a.tx_chunk = plan.lp.tx_chunk;
-            a.channel = channel_data;
-            a.arrivals = tx_wave_arrivals_s;
-            a.out = out;
-            a.n_tx = static_cast<int32_t>(n_tx);
-            a.accumulate = 1;
-            a.power = 1;
-            if (overwrite) MACH_B200_CUDA_TRY(cudaMemsetAsync(out, 0, power_bytes, stream));
-            if ((rc = dispatch_split(storage, a, interp_type, plan, stream))) return rc;
-            if (!(flags & MACH_B200_FLAG_ASYNC)) {
-                MACH_B200_CUDA_TRY(cudaStreamSynchronize(stream));
-                return check_status(dev, stream);
-            }
-            return MACH_B200_OK;
+        if (!(plan.ensemble || plan.frame_lane) || per_tx * n_tx >= (int64_t{1} << 31)) return MACH_B200_OK;
+        *fused = true;
+        plan.st.status = dev->status;
+        DasArgs a = make_args(rx_coords_m, scan_coords_m, n_scan, n_rx, n_samples, n_frames, f_number, rx_start_s,
+                              sampling_freq_hz, sound_speed_m_s, modulation_freq_hz, tukey_alpha, channel_scale,
+                              cplx, flags);
+        a.frame_passes = plan.lp.passes;
+        a.tx_chunk = plan.lp.tx_chunk;
+        a.channel = channel_data;
+        a.arrivals = tx_wave_arrivals_s;
+        a.out = out;
+        a.n_tx = static_cast<int32_t>(n_tx);
+        a.accumulate = 1;
+        a.power = 1;
+        if (overwrite) MACH_B200_CUDA_TRY(cudaMemsetAsync(out, 0, power_bytes, stream));
+        const int rc2 = dispatch_split(storage, a, interp_type, plan, stream);
+        if (rc2) return rc2;
+        if (!(flags & MACH_B200_FLAG_ASYNC)) {
+            MACH_B200_CUDA_TRY(cudaStreamSynchronize(stream));
+            return check_status(dev, stream);
         }
-    }
+        return MACH_B200_OK;
+    };
+    bool fused = false;
+    rc = run_fused(opt, &fused);
+    if (rc || fused) return rc;
 
-    // ---- general: full image into a temporary buffer, then the reduction kernel
+    // ---- general: full image into a temporary buffer, then the reduction kernel.  Where the image
+    // does not fit, the ensemble kernel, which needs none, if it takes the job.
     const size_t image_bytes = static_cast<size_t>(n_scan) * n_frames * (cplx ? 8 : 4);
     DeviceBuffer image, power;
-    MACH_B200_CUDA_TRY(image.alloc(image_bytes, stream));
+    const cudaError_t image_error = image.alloc(image_bytes, stream);
+    if (image_error != cudaSuccess) {
+        cudaGetLastError();
+        mach_b200_options ensemble = opt;
+        ensemble.kernel = MACH_B200_KERNEL_ENSEMBLE;
+        rc = run_fused(ensemble, &fused);
+        if (rc || fused) return rc;
+        MACH_B200_CUDA_TRY(image_error);
+    }
     mach_b200_options o = opt;
     o.flags = (flags & ~(MACH_B200_FLAG_POWER_DOPPLER | MACH_B200_FLAG_ASYNC)) | MACH_B200_FLAG_OVERWRITE;
     if (all_device && (flags & MACH_B200_FLAG_ASYNC)) o.flags |= MACH_B200_FLAG_ASYNC;
