@@ -38,8 +38,8 @@ def candidates(storage: str, n_frames: int, grid: Any) -> list[dict]:
     vf = 8 // esz
     out: list[dict] = []
     grids = [None, False] if grid else [False]
-    if n_frames > 16 and n_frames % 8 == 0:  # the voxel-per-lane kernel in 8-frame chunks
-        for tile_fast in ((2, 4) if grid else (0,)):
+    if n_frames > 16 and n_frames % 8 == 0:  # the voxel-per-lane and frame-group kernels in chunks of frames
+        for tile_fast in ((1, 2, 4) if grid else (0,)):
             out.append({"kernel": "lane_voxel", "tile_fast": tile_fast})
     if n_frames <= 8 or n_frames == 16:
         for tx_chunk in (8, 16, 32, 40):
@@ -174,7 +174,10 @@ def tune(channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, *, reps: 
                           device=channel_data.device)
     stream = torch.cuda.current_stream()
     best, best_ms, timings = None, float("inf"), []
-    for cand in candidates(storage, n_frames, grid):
+    cands = candidates(storage, n_frames, grid)
+    if any(c["kernel"] == "lane_voxel" for c in cands):
+        cands.insert(0, {"kernel": "lane_voxel"})  # with its own choice of every knob
+    for cand in cands:
         kw = dict(cand)
 
         def run():
