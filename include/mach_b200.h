@@ -80,7 +80,8 @@ extern "C" {
 
 /* Kernel families (mach_b200_options.kernel). */
 #define MACH_B200_KERNEL_AUTO 0
-#define MACH_B200_KERNEL_LANE_VOXEL 1 /* one lane per voxel, all frames in registers (1..8 frames) */
+#define MACH_B200_KERNEL_LANE_VOXEL 1 /* one lane per voxel, frames in registers (1..8, or chunks of 8 and 16);
+                                         more than 8 complex frames: groups of 2..16 lanes per voxel */
 #define MACH_B200_KERNEL_STAGED 2     /* voxel tiles, sample windows staged in shared memory by TMA */
 #define MACH_B200_KERNEL_WARP 3       /* a warp per voxel over frames, taps read from global memory */
 #define MACH_B200_KERNEL_ENSEMBLE 4   /* lanes = frames of a 32-lane block, voxel-tile sample windows in
