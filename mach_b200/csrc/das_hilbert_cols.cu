@@ -21,8 +21,8 @@
 //
 // Bound: the 12 bytes per sample of HBM traffic are 59 us for the compounding acquisition
 // (32 M samples of 3328 = 16 16 13); instruction issue and the shared-memory round trips follow.
-// Measured on B200 for that job: 0.52 ms out of place -> 0.22 ms in place (staging the next group with cp.async: 0.24 ms;
-// three CTAs per SM without x in registers: 0.28 ms).
+// Measured on B200 for that job: 0.52 ms out of place -> 0.22 ms in place (staging the next group with
+// cp.async: 0.24 ms; three CTAs per SM without x in registers: 0.28 ms).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 

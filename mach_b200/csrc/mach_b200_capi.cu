@@ -1448,7 +1448,6 @@ int hilbert_impl(int32_t src_storage, const void* src, int32_t src_layout, int32
     const bool planned = F == 1 && hilbert_cols_plan(g.n, h);
     h.pair_vec = src_storage == kF32 && src_layout == MACH_B200_LAYOUT_ACQUISITION && n_cols % 2 == 0 &&
                  reinterpret_cast<uintptr_t>(g.src) % 8 == 0;
-    if (planned && hilbert_cols_smem(h) > static_cast<size_t>(max_smem) - 4096) h.pair_vec = 0;
     if (planned && hilbert_cols_smem(h) <= static_cast<size_t>(max_smem) - 4096) {
         h.src = g.src;
         h.dst = dst;
