@@ -473,7 +473,8 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
                 const int64_t per_outer = vpc >> lw;
                 const int64_t tiles = ((lp.map_outer + per_outer - 1) / per_outer) * ((lp.map_fast + wf - 1) / wf);
                 lp.grid = dim3(static_cast<unsigned>(tiles), 1, 1);
-            } else if (probe && n_frames > 8) {
+            } else if (probe && n_frames > 8 && !grid_matches(o, n_vox)) {
+                // (only where the caller names no grid: then every launch of the plan probes, or none)
                 lp.probe_grid = true;
                 lp.map_wlog = lw;
                 lp.tile_rev = rev;
