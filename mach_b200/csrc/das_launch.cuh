@@ -49,11 +49,13 @@ struct LaunchPlan {
     int run_voxels;     // frame-lane kernel: G, voxels per warp run (J * G = 16)
 };
 
-// Opt a kernel into more than 48 KB of dynamic shared memory (once per instance is enough,
-// repeating it is harmless).
+// Opt a kernel into more than 48 KB of shared memory, which its static arrays (no kernel that asks has
+// kStaticSmem of them) and its dynamic ones share (once per instance is enough, repeating it is
+// harmless).
+constexpr size_t kStaticSmem = 4 * 1024;
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
-    if (bytes <= 48 * 1024) return cudaSuccess;
+    if (bytes + kStaticSmem <= 48 * 1024) return cudaSuccess;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
 }
 
