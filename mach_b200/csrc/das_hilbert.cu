@@ -468,7 +468,7 @@ cudaError_t hilbert_typed(const HilbertArgs& g, size_t smem, cudaStream_t st) {
     bool odd = false;
     for (int s = 0; s < g.n_stages; ++s) odd = odd || (g.radix[s] & (g.radix[s] - 1)) != 0;
     auto k = odd ? hilbert_kernel<In, Out, true> : hilbert_kernel<In, Out, false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     int device = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;

@@ -538,7 +538,7 @@ cudaError_t launch_hilbert_cols(const HilbertColsArgs& g, cudaStream_t st) {
     const size_t smem = hilbert_cols_smem(g);
     const bool keep = (g.low[0] << g.pairs_log2) <= kThreads;
     auto k = keep ? hilbert_cols_kernel<true> : hilbert_cols_kernel<false>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    cudaError_t e = allow_smem(k, smem);
     if (e != cudaSuccess) return e;
     int device = 0, sms = 0, per_sm = 0;
     if ((e = cudaGetDevice(&device)) != cudaSuccess) return e;

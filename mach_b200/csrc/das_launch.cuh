@@ -49,14 +49,23 @@ struct LaunchPlan {
     int run_voxels;     // frame-lane kernel: G, voxels per warp run (J * G = 16)
 };
 
-// Opt a kernel into more than 48 KB of shared memory, which its static arrays (no kernel that asks has
-// kStaticSmem of them) and its dynamic ones share (once per instance is enough, repeating it is
-// harmless).
+// Opt a kernel into more than 48 KB of shared memory, where its static arrays (no kernel that asks has
+// kStaticSmem of them) and the dynamic ones together may need it.  The limit is set to all that a
+// block can have, whatever this launch needs: it is one value per kernel and device, so threads that
+// launch the same kernel with different sizes do not lower each other's.
 constexpr size_t kStaticSmem = 4 * 1024;
 template <typename K>
 cudaError_t allow_smem(K kernel, size_t bytes) {
     if (bytes + kStaticSmem <= 48 * 1024) return cudaSuccess;
-    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes));
+    cudaFuncAttributes fa{};
+    int device = 0, block = 0;
+    cudaError_t e = cudaFuncGetAttributes(&fa, kernel);
+    if (e == cudaSuccess) e = cudaGetDevice(&device);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    if (e != cudaSuccess) return e;
+    const int limit = block - static_cast<int>(fa.sharedSizeBytes);
+    if (fa.maxDynamicSharedSizeBytes == limit) return cudaSuccess;
+    return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit);
 }
 
 template <int S, int I, int LV>
