@@ -1602,7 +1602,9 @@ int noalloc_impl(int32_t storage, const void* channel_data, const float* rx_coor
 struct mach_b200_batch {
     int device = 0;
     uint32_t max_jobs = 0;
-    static constexpr int kMaxGroups = 64;
+    // Complex ensembles have 120 signatures (4 storages, 3 interpolations, 2 delay modes, 5 lane counts), of
+    // which one job may take three; the rest leaves room for every other kernel that a batch meets.
+    static constexpr int kMaxGroups = 256;
     static constexpr uint32_t kMaxParts = 1 + kMaxRest;  // launches of one job
     // pinned host tables (filled on the host, copied by the stream)
     BatchJob* h_jobs = nullptr;
