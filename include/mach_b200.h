@@ -271,7 +271,7 @@ typedef struct mach_b200_job {
     const float* rx_coords_m;    /* [n_rx][3] */
     const float* scan_coords_m;  /* [n_scan][3] */
     const float* tx_wave_arrivals_s; /* [n_tx][n_scan] */
-    void* out;                   /* [n_scan][n_frames] */
+    void* out;                   /* [n_scan][n_frames]; jobs that share it: see mach_b200_batch_run */
     uint32_t n_tx, n_rx, n_samples, n_frames;
     uint64_t n_scan;
     float f_number, rx_start_s, sampling_freq_hz, sound_speed_m_s, modulation_freq_hz, tukey_alpha;
@@ -294,9 +294,13 @@ MACH_B200_API int mach_b200_batch_create(uint32_t max_jobs, mach_b200_batch** ba
  * Beamform a batch of device-resident jobs with one persistent launch per kernel
  * signature (storage, interpolation, kernel family): the resident CTAs pull (job, tile)
  * work items from a device counter until every tile of every job is done, so jobs of
- * different grid sizes, transmit and frame counts share the GPU.  Only asynchronous
- * copies (job table, from the context's pinned buffer), memsets and launches are
- * enqueued on `cuda_stream`, so the call can be captured in a CUDA graph and replayed
+ * different grid sizes, transmit and frame counts share the GPU.  Launches of different
+ * signatures run side by side, on streams that fork from `cuda_stream` and join it again, unless
+ * a job writes a buffer that another job writes or reads: then they run one after the other, in the
+ * order of their first jobs (two jobs of different signatures may add into one image).  Jobs of
+ * one signature always share a launch and must not share an output.  Only asynchronous
+ * copies (job table, from the context's pinned buffer), memsets, event waits and launches are
+ * enqueued, so the call can be captured in a CUDA graph and replayed
  * (replays reuse the captured job table).  mach has no batch interface (its call
  * beamforms one transmit of one job), so this entry point has no counterpart there.
  * `flags`: MACH_B200_FLAG_ASYNC to return without synchronising.

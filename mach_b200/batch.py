@@ -69,7 +69,9 @@ class Job:
 
     ``channel`` is ``[n_tx, n_rx, n_samples, n_frames]`` (or ``[..., 2]`` (I, Q) pairs of a
     16-bit type), ``arrivals`` ``[n_tx, n_scan]``; ``out`` is allocated when omitted and is
-    overwritten (``accumulate=True`` adds into it instead).
+    overwritten (``accumulate=True`` adds into it instead).  Jobs that share an ``out``, or of which
+    one reads another's, run in order when their kernel signatures (storage, interpolation, frame
+    class, delay mode) differ; jobs of one signature share a launch and must not.
     """
 
     channel: Any

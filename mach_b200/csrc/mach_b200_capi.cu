@@ -15,6 +15,7 @@
 #include <vector>
 
 #include "das_launch.cuh"
+#include "das_overlap.h"
 #include "das_split.h"
 #include "das_tiles.h"
 #include "mach_b200.h"
@@ -1617,8 +1618,8 @@ struct mach_b200_batch {
     unsigned long long* d_counters = nullptr;
     cudaEvent_t copied = nullptr;  // host tables may be rewritten once this has passed
     bool pending = false;
-    // The launches of one run are independent: they go to the caller's stream and these, forked
-    // from it and joined to it again, so that one launch's last tiles run beside the next one's
+    // Where no job writes what another one writes or reads, the launches of one run are independent:
+    // they go to the caller's stream and these, forked from it and joined to it again, so that one launch's last tiles run beside the next one's
     // first (five launches of a mixed batch on B200: 744 us one after the other, 623 us so).
     static constexpr int kSideStreams = 3;
     cudaStream_t side[kSideStreams] = {};
@@ -1804,6 +1805,17 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
     std::vector<int64_t> items(n_groups, 0);
     std::vector<int> max_items(n_groups, 0);
     std::vector<double> points(n_groups, 0.0);
+    std::vector<JobRange> written, read;
+    for (uint32_t i = 0; i < n_jobs; ++i) {
+        const mach_b200_job& j = jobs[i];
+        const uint64_t sums = j.n_scan * j.n_frames, samples = static_cast<uint64_t>(j.n_rx) * j.n_samples * j.n_frames;
+        add_range(written, j.out, sums * ((j.storage & 1) ? 8 : 4), i);
+        add_range(read, j.channel_data, j.n_tx * samples * storage_bytes(j.storage), i);
+        add_range(read, j.rx_coords_m, uint64_t{12} * j.n_rx, i);
+        add_range(read, j.scan_coords_m, 12 * j.n_scan, i);
+        add_range(read, j.tx_wave_arrivals_s, 4 * j.n_scan * j.n_tx, i);
+    }
+    const bool in_order = jobs_share_outputs(written, read);
     for (const Part& part : parts) {
         const mach_b200_job& j = jobs[part.job];
         const int g = part.group;
@@ -1862,12 +1874,14 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         }
     }
     bool any_waits = false;  // staged kernels have bounded waits
-    std::vector<int> order;  // the groups with work, most points first
+    // The groups with work, most points first; where jobs share outputs, in job order on the caller's
+    // stream alone.
+    std::vector<int> order;
     for (int g = 0; g < n_groups; ++g) {
         if (items[g] > 0) order.push_back(g);
     }
-    std::sort(order.begin(), order.end(), [&](int x, int y) { return points[x] > points[y]; });
-    const int n_side = std::min<int>(mach_b200_batch::kSideStreams, static_cast<int>(order.size()) - 1);
+    if (!in_order) std::sort(order.begin(), order.end(), [&](int x, int y) { return points[x] > points[y]; });
+    const int n_side = in_order ? 0 : std::min<int>(mach_b200_batch::kSideStreams, static_cast<int>(order.size()) - 1);
     if (n_side > 0) MACH_B200_CUDA_TRY(cudaEventRecord(b->forked, stream));
     for (int i = 0; i < n_side; ++i) MACH_B200_CUDA_TRY(cudaStreamWaitEvent(b->side[i], b->forked, 0));
     cudaError_t launched = cudaSuccess;
