@@ -21,7 +21,9 @@ def is_contiguous(array: Any) -> bool:
 
 
 def ensure_contiguous(array: Any, *, warn: bool = True) -> Any:
-    """Return a C-contiguous array, warning when a copy is made (src/mach/_check.py:25-41)."""
+    """Return a C-contiguous array, warning when a copy is made (src/mach/_check.py:25-41).  Views that
+    torch conjugates or negates lazily are resolved."""
+    array = _dlpack.resolved(array)
     if is_contiguous(array):
         return array
     if warn:

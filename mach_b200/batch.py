@@ -114,8 +114,8 @@ class Job:
     def as_struct(self) -> _Job:
         for name in ("channel", "rx_coords_m", "scan_coords_m", "arrivals", "out"):
             t = getattr(self, name)
-            if not (t.is_cuda and t.is_contiguous()):
-                raise ValueError(f"Job.{name} must be a contiguous CUDA tensor")
+            if not (t.is_cuda and t.is_contiguous()) or _dlpack.is_lazy(t):
+                raise ValueError(f"Job.{name} must be a contiguous CUDA tensor (not lazily conjugated or negated)")
         n_tx, n_rx, n_s, n_f = (int(d) for d in self.channel.shape[:4])
         j = _Job()
         j.storage = _cuda_impl.STORAGE_CODES[self.storage]

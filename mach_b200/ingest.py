@@ -11,7 +11,7 @@ from __future__ import annotations
 
 from typing import Any
 
-from mach_b200 import _cuda_impl
+from mach_b200 import _cuda_impl, _dlpack
 
 _lib = _cuda_impl._lib
 
@@ -75,9 +75,9 @@ def ingest(signal: Any, storage: str | None = None, *, scale: float = 1.0, compl
     shape = (n_w, n_e, n_s, n_f) + ((2,) if pairs_out else ())
     if out is None:
         out = torch.empty(shape, dtype=getattr(torch, dt_name), device="cuda")
-    elif tuple(out.shape) != shape or not out.is_cuda or not out.is_contiguous():
+    elif tuple(out.shape) != shape or not out.is_cuda or not out.is_contiguous() or _dlpack.is_lazy(out):
         raise ValueError(f"out must be a contiguous CUDA tensor of shape {list(shape)}")
-    sig = signal.contiguous()
+    sig = _dlpack.resolved(signal).contiguous()
     stream = torch.cuda.current_stream().cuda_stream
     flags = 0 if (sync or not sig.is_cuda) else _cuda_impl.FLAG_ASYNC
     rc = _lib.mach_b200_ingest(_cuda_impl.STORAGE_CODES[src], sig.data_ptr(), _cuda_impl.STORAGE_CODES[dst],
@@ -136,9 +136,10 @@ def hilbert(signal: Any, storage: str | None = None, *, layout: str = "channel",
     shape = (n_w, n_e, n_s, n_f) + ((2,) if pairs_out else ())
     if out is None:
         out = torch.empty(shape, dtype=getattr(torch, dt_name), device="cuda")
-    elif tuple(out.shape) != shape or not out.is_cuda or not out.is_contiguous() or out.dtype != getattr(torch, dt_name):
+    elif (tuple(out.shape) != shape or not out.is_cuda or not out.is_contiguous() or _dlpack.is_lazy(out)
+          or out.dtype != getattr(torch, dt_name)):
         raise ValueError(f"out must be a contiguous CUDA {dt_name} tensor of shape {list(shape)}")
-    sig = signal.contiguous()
+    sig = _dlpack.resolved(signal).contiguous()
     stream = torch.cuda.current_stream().cuda_stream
     flags = 0 if (sync or not sig.is_cuda) else _cuda_impl.FLAG_ASYNC
     code = _cuda_impl.LAYOUT_CHANNEL if layout == "channel" else _cuda_impl.LAYOUT_ACQUISITION

@@ -44,7 +44,7 @@ def _plain_tensors(channel_data: Any, rx_coords_m: Any, scan_coords_m: Any, tx_w
         return False
     tensor, f32 = torch.Tensor, torch.float32
     for x in (channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s):
-        if type(x) is not tensor or not x.is_cuda or not x.is_contiguous():
+        if type(x) is not tensor or not x.is_cuda or not x.is_contiguous() or x.is_conj() or x.is_neg():
             return False
     dtype = channel_data.dtype
     if dtype is not f32 and dtype is not torch.complex64:
@@ -56,7 +56,7 @@ def _plain_tensors(channel_data: Any, rx_coords_m: Any, scan_coords_m: Any, tx_w
             scan_coords_m.shape != (*n_scan, 3) or tx_wave_arrivals_s.shape != n_scan):
         return False
     return out is None or (type(out) is tensor and out.is_cuda and out.dtype is dtype and out.is_contiguous()
-                           and out.shape == (*n_scan, shape[2]))
+                           and not out.is_conj() and not out.is_neg() and out.shape == (*n_scan, shape[2]))
 
 
 def beamform(
@@ -167,6 +167,8 @@ def beamform(
         raise ValueError("Output array `out` is not writable. Try using cupy or pytorch for the output array.")
     if not is_contiguous(out):
         raise ValueError("Output array `out` must be contiguous.")
+    if _dlpack.is_lazy(out):
+        raise ValueError("Output array `out` must not be a lazily conjugated or negated view.")
 
     nb_beamform(
         channel_data,
