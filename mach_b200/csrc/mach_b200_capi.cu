@@ -130,6 +130,14 @@ int residency(const void* p, int device, Residency* r, const char* name) {
 
 constexpr int kMaxDevices = 64;
 
+// A stream that part of a batch runs on beside the caller's, with the event that forks or joins it.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    cudaEvent_t event = nullptr;
+    int priority = 0;
+};
+constexpr int kMaxSideStreams = 24;  // per device, all batches and threads together
+
 struct DeviceState {
     std::once_flag once;
     cudaError_t init_error = cudaSuccess;
@@ -137,6 +145,9 @@ struct DeviceState {
     std::once_flag pool_once;
     cudaError_t pool_error = cudaSuccess;
     std::atomic<cudaMemPool_t> pool{nullptr};  // the library's own stream-ordered pool for staging buffers
+    std::mutex side_mutex;
+    std::vector<SideStream> side_free;  // least recently used first
+    int side_total = 0;
 };
 DeviceState g_devices[kMaxDevices];
 
@@ -183,6 +194,67 @@ cudaError_t library_pool(int device, cudaMemPool_t* pool) {
     *pool = d.pool.load();
     return d.pool_error;
 }
+
+// Up to `n` side streams of the caller's priority for the time of one batch run, from the device's
+// list; they go back when it has enqueued its work.  Batches make none of their own (three streams
+// and events cost 160 us to make and as much to destroy, more than one run gains by them).  A stream
+// with work still on it is taken only when no further one may be made: it would tie two batches
+// together.  A stream that takes part in a graph capture goes back with the capture still open
+// and is passed over until that has ended.
+struct SideStreams {
+    DeviceState* dev = nullptr;
+    std::vector<SideStream> taken;
+    SideStreams() = default;
+    SideStreams(const SideStreams&) = delete;
+    SideStreams& operator=(const SideStreams&) = delete;
+    ~SideStreams() {
+        if (taken.empty()) return;
+        std::lock_guard<std::mutex> lock(dev->side_mutex);
+        dev->side_free.insert(dev->side_free.end(), taken.begin(), taken.end());
+    }
+    void take(DeviceState* d, cudaStream_t caller, int n) {
+        if (n <= 0) return;
+        dev = d;
+        int priority = 0;
+        cudaStreamGetPriority(caller, &priority);
+        // (queries and stream creation must not disturb a capture of this or another thread)
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        {
+            std::lock_guard<std::mutex> lock(d->side_mutex);
+            d->side_free.reserve(kMaxSideStreams);  // the way back allocates nothing
+            for (int pass = 0; pass < 2; ++pass) {  // idle streams and new ones, then busy ones
+                for (size_t i = 0; i < d->side_free.size() && static_cast<int>(taken.size()) < n;) {
+                    const SideStream s = d->side_free[i];
+                    cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
+                    const bool usable = s.priority == priority &&
+                                        cudaStreamIsCapturing(s.stream, &status) == cudaSuccess &&
+                                        status == cudaStreamCaptureStatusNone &&
+                                        (pass == 1 || cudaStreamQuery(s.stream) == cudaSuccess);
+                    if (!usable) {
+                        ++i;
+                        continue;
+                    }
+                    taken.push_back(s);
+                    d->side_free.erase(d->side_free.begin() + static_cast<std::ptrdiff_t>(i));
+                }
+                while (pass == 0 && static_cast<int>(taken.size()) < n && d->side_total < kMaxSideStreams) {
+                    SideStream s;
+                    s.priority = priority;
+                    if (cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, priority) != cudaSuccess) break;
+                    if (cudaEventCreateWithFlags(&s.event, cudaEventDisableTiming) != cudaSuccess) {
+                        cudaStreamDestroy(s.stream);
+                        break;
+                    }
+                    ++d->side_total;
+                    taken.push_back(s);
+                }
+            }
+        }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        cudaGetLastError();  // a query's "not ready", or no room for a further stream: the run needs none
+    }
+};
 
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
@@ -1619,11 +1691,10 @@ struct mach_b200_batch {
     cudaEvent_t copied = nullptr;  // host tables may be rewritten once this has passed
     bool pending = false;
     // Where no job writes what another one writes or reads, the launches of one run are independent:
-    // they go to the caller's stream and these, forked from it and joined to it again, so that one launch's last tiles run beside the next one's
-    // first (five launches of a mixed batch on B200: 744 us one after the other, 623 us so).
+    // they go to the caller's stream and up to so many side streams, forked from it and joined again,
+    // so that one launch's last tiles run beside the next one's first (five launches of a mixed batch
+    // on B200: 744 us one after the other, 623 us so).
     static constexpr int kSideStreams = 3;
-    cudaStream_t side[kSideStreams] = {};
-    cudaEvent_t forked = nullptr, joined[kSideStreams] = {};
 };
 
 namespace {
@@ -1671,11 +1742,6 @@ void batch_free(mach_b200_batch* b) {
         cudaEventSynchronize(b->copied);
         cudaEventDestroy(b->copied);
     }
-    for (int i = 0; i < mach_b200_batch::kSideStreams; ++i) {
-        if (b->side[i]) cudaStreamDestroy(b->side[i]);
-        if (b->joined[i]) cudaEventDestroy(b->joined[i]);
-    }
-    if (b->forked) cudaEventDestroy(b->forked);
     cudaFreeHost(b->h_jobs);
     cudaFreeHost(b->h_begin);
     cudaFreeHost(b->h_hdr);
@@ -1703,11 +1769,6 @@ int batch_create(uint32_t max_jobs, mach_b200_batch** out) {
     if (e == cudaSuccess) e = cudaMalloc(&b->d_hdr, sizeof(BatchHeader) * G);
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counters, sizeof(unsigned long long) * G);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->copied, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->forked, cudaEventDisableTiming);
-    for (int i = 0; i < mach_b200_batch::kSideStreams; ++i) {
-        if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->side[i], cudaStreamNonBlocking);
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->joined[i], cudaEventDisableTiming);
-    }
     if (e != cudaSuccess) {
         batch_free(b);
         return fail(MACH_B200_ERR_CUDA, "batch context allocation failed: %s", cudaGetErrorString(e));
@@ -1881,20 +1942,22 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
         if (items[g] > 0) order.push_back(g);
     }
     if (!in_order) std::sort(order.begin(), order.end(), [&](int x, int y) { return points[x] > points[y]; });
-    const int n_side = in_order ? 0 : std::min<int>(mach_b200_batch::kSideStreams, static_cast<int>(order.size()) - 1);
-    if (n_side > 0) MACH_B200_CUDA_TRY(cudaEventRecord(b->forked, stream));
-    for (int i = 0; i < n_side; ++i) MACH_B200_CUDA_TRY(cudaStreamWaitEvent(b->side[i], b->forked, 0));
+    SideStreams sides;
+    if (!in_order) sides.take(dev, stream, std::min<int>(mach_b200_batch::kSideStreams, static_cast<int>(order.size()) - 1));
+    const int n_side = static_cast<int>(sides.taken.size());
+    if (n_side > 0) MACH_B200_CUDA_TRY(cudaEventRecord(sides.taken[0].event, stream));
+    for (const SideStream& s : sides.taken) MACH_B200_CUDA_TRY(cudaStreamWaitEvent(s.stream, sides.taken[0].event, 0));
     cudaError_t launched = cudaSuccess;
     for (size_t k = 0; k < order.size() && launched == cudaSuccess; ++k) {
         const int g = order[k], lane = static_cast<int>(k) % (n_side + 1);
         PersistentLaunch pl{b->d_hdr + g, b->d_jobs + first[g], b->d_begin + first[g], b->d_counters + g, smem[g],
                             max_items[g]};
         any_waits |= keys[g].family == 1;
-        launched = launch_group(keys[g], pl, lane == 0 ? stream : b->side[lane - 1]);
+        launched = launch_group(keys[g], pl, lane == 0 ? stream : sides.taken[lane - 1].stream);
     }
-    for (int i = 0; i < n_side; ++i) {  // joined also after a failed launch
-        MACH_B200_CUDA_TRY(cudaEventRecord(b->joined[i], b->side[i]));
-        MACH_B200_CUDA_TRY(cudaStreamWaitEvent(stream, b->joined[i], 0));
+    for (const SideStream& s : sides.taken) {  // joined also after a failed launch
+        MACH_B200_CUDA_TRY(cudaEventRecord(s.event, s.stream));
+        MACH_B200_CUDA_TRY(cudaStreamWaitEvent(stream, s.event, 0));
     }
     MACH_B200_CUDA_TRY(launched);
     if (!(flags & MACH_B200_FLAG_ASYNC)) {
