@@ -510,7 +510,10 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
         kind = n_frames <= 8 || chunks_ok ? MACH_B200_KERNEL_LANE_VOXEL
                                           : (vec_ok ? MACH_B200_KERNEL_STAGED : MACH_B200_KERNEL_WARP);
     }
-    if (kind == MACH_B200_KERNEL_LANE_VOXEL && n_frames > 8 && !chunks_ok) kind = MACH_B200_KERNEL_WARP;
+    // (a batch has neither padded copies nor the warp kernel: knobs tuned on single calls still run there)
+    if (kind == MACH_B200_KERNEL_LANE_VOXEL && n_frames > 8 && !chunks_ok) {
+        kind = batch ? MACH_B200_KERNEL_STAGED : MACH_B200_KERNEL_WARP;
+    }
     if (kind == MACH_B200_KERNEL_STAGED && !vec_ok) kind = MACH_B200_KERNEL_WARP;
 
     if (kind == MACH_B200_KERNEL_LANE_VOXEL) {

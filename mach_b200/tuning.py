@@ -38,7 +38,7 @@ def candidates(storage: str, n_frames: int, grid: Any) -> list[dict]:
     vf = 8 // esz
     out: list[dict] = []
     grids = [None, False] if grid else [False]
-    if n_frames > 16 and n_frames % 8 == 0:  # the voxel-per-lane and frame-group kernels in chunks of frames
+    if n_frames > 8 and n_frames != 16:  # the voxel-per-lane and frame-group kernels in chunks of frames
         for tile_fast in ((1, 2, 4) if grid else (0,)):
             out.append({"kernel": "lane_voxel", "tile_fast": tile_fast})
     if n_frames <= 8 or n_frames == 16:
@@ -74,6 +74,16 @@ def candidates(storage: str, n_frames: int, grid: Any) -> list[dict]:
         out.append({"kernel": "warp"})
     return out
 
+
+def plain_candidates(storage: str, n_frames: int, grid: Any) -> list[dict]:
+    """Every family of :func:`candidates` with its own choice of every knob.  The launch of an untuned
+    automatic call is one of them, so that a tuned call is never slower than that by what was timed."""
+    return [{"kernel": k} for k in dict.fromkeys(c["kernel"] for c in candidates(storage, n_frames, grid))]
+
+
+# Part of every cache key: entries that were timed on other kernels, or on other rules for choosing
+# them, are not used.  Raised when either changes.
+KERNEL_SET = 2
 
 _DEVICE_NAMES: dict[int, str] = {}
 _LOADED = False
@@ -115,7 +125,7 @@ def lookup(storage, n_tx, n_rx, n_samples, n_frames, n_vox, grid, interp, device
 
 def _key(storage, n_tx, n_rx, n_samples, n_frames, n_vox, grid, interp, device_name, delay="auto") -> str:
     return (f"{device_name}|{storage}|tx{n_tx}|rx{n_rx}|s{n_samples}|f{n_frames}|v{n_vox}|g{grid}|i{int(interp)}"
-            f"|d{delay}")
+            f"|d{delay}|k{KERNEL_SET}")
 
 
 def _load() -> dict:
@@ -174,10 +184,7 @@ def tune(channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, *, reps: 
                           device=channel_data.device)
     stream = torch.cuda.current_stream()
     best, best_ms, timings = None, float("inf"), []
-    cands = candidates(storage, n_frames, grid)
-    if any(c["kernel"] == "lane_voxel" for c in cands):
-        cands.insert(0, {"kernel": "lane_voxel"})  # with its own choice of every knob
-    for cand in cands:
+    for cand in plain_candidates(storage, n_frames, grid) + candidates(storage, n_frames, grid):
         kw = dict(cand)
 
         def run():
