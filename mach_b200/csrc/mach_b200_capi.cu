@@ -581,10 +581,9 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
             p.lp.pad_frames = !rows_ok && !real8_ok ? static_cast<int>(padded) : 0;
         } else {
             // Groups of 16, 8, 4 and 2 lanes take 128, 64, 32 and 16 frames of a voxel; the more, the
-            // cheaper a frame (das_frame_group.cuh), so the frames go to the widest group first, with
-            // a partly empty chunk where at least three quarters of it are used, and the last 8 to the
-            // one-lane kernel.  24 frames alone run as three chunks of that kernel (complex64 295 us
-            // against 309 us and 324 us with 2 and 4 lanes).  Warps lie across the contiguous axis for
+            // cheaper a frame (das_frame_group.cuh), so on a large scan the frames go to the widest
+            // group first, with a partly empty chunk where more than three quarters of it are used (of 4
+            // lanes: three quarters), and the last 8 to the one-lane kernel.  Warps lie across the contiguous axis for
             // complex64 (fewest rows: 192 frames with 4 lanes 2.93 / 3.01 ms with 1 / 2 voxels along
             // it); 4-byte pairs are within 2 %.
             int n = 0;
@@ -597,14 +596,43 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
                 at += 8u * lanes * chunks;
                 left = padded > at ? padded - at : 0;
             };
-            if (padded == 24) {
-                add(1, 3);
-            } else {
-                add(16, (left + 31) / 128);
-                add(8, (left + 15) / 64);
-                add(4, (left + 8) / 32);
-                add(2, left / 16);
-                add(1, left / 8);
+            add(16, (left + 31) / 128);
+            add(8, (left + 15) / 64);
+            add(4, (left + 8) / 32);
+            add(2, left / 16);
+            add(1, left / 8);
+            // On a small scan each launch leaves the GPU partly idle, and the narrow ones take as long as
+            // the wide one, so all frames go into one launch, of the widest groups.  Measured on B200,
+            // three launches / one of 16 lanes, 200 complex64 frames: 256 points x 1 transmit 268 / 95 us,
+            // x 5 1.85 / 0.60 ms; 16384 points 315 / 205 us and 1.36 / 0.85 ms; 32768 points 0.40 / 0.34
+            // and 1.59 / 1.39 ms, but 0.70 / 0.71 and 3.76 / 4.28 ms for points in random order; 65536
+            // points 0.57 / 0.59 and 2.24 / 2.51 ms.  136 frames (6 % of the last chunk used): 16384
+            // points 226 / 195 us, 32768 points 300 / 326 us.  8 lanes for at most 64 frames above 8192
+            // points: 40 frames on 16384 points 113 us against 118 us and 184 us in two launches.
+            const bool half_used = padded % 128 == 0 || padded % 128 > 64;
+            // (24 pairs of 4 bytes: groups of 4 lanes from 4096 points on, int16 8192 points in random order x 5
+            // transmits 372 us against 481 us)
+            const uint64_t small_scan = esz == 8 ? 16384 : (padded == 24 ? 4096 : (half_used ? 32768 : 16384));
+            const bool several = n > 1 || padded == 24;
+            if (several && n_vox <= small_scan) {
+                n = 0;
+                at = 0;
+                const uint32_t lanes = padded <= 64 && n_vox > 8192 ? 8 : 16;
+                add(static_cast<int>(lanes), (padded + 8 * lanes - 1) / (8 * lanes));
+            } else if (padded == 24) {
+                // complex64 as three one-lane chunks (256 x 256 points x 5 transmits 432 / 481 us with
+                // 1 / 4 lanes), pairs of 4 bytes in groups of 4 lanes (FP16 pairs 351 / 328 us)
+                n = 0;
+                at = 0;
+                if (esz == 8) add(1, 3);
+                else add(4, 1);
+            } else if (several && padded <= 48 && n_vox <= 65536) {
+                // 40 and 48 frames: two-lane chunks alone (40 frames, 32768 points x 5 transmits 752 -> 449 us
+                // for complex64, 514 -> 369 us for FP16 pairs; 65536 points 721 -> 670 and 604 -> 560 us;
+                // 160000 points 1.21 -> 1.46 ms)
+                n = 0;
+                at = 0;
+                add(2, padded / 16 + (padded % 16 != 0));
             }
             p.lp = parts[0];
             for (int k = 1; k < n; ++k) p.rest[p.n_rest++] = parts[k];
