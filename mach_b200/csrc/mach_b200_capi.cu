@@ -455,6 +455,25 @@ bool pad_fits(uint32_t n_rx, uint32_t n_samples, uint32_t n_tx, uint32_t padded,
     return per_tx * esz <= kPadBytes / n_tx;
 }
 
+// Whether the copy pays where the staged kernel cannot read the rows either.  The alternative is the warp
+// kernel, slow per point, but with no copy, whose cost goes with the samples, and full GPU use from few
+// voxels.  Measured on B200 with 128 elements, warp kernel / padded copy, at the last size below each line and
+// the first above it:
+//   9 FP16 pairs, 1000 samples x 5 transmits: 12288 points 303 / 269 us, 4000 x 3: 209 / 249 us; 20480
+//     points 421 / 270 and 283 / 241 us (9 float32 frames 341 / 242 and 232 / 232 us)
+//   17 FP16 pairs (wide frame groups need fewer voxels), 1500 x 5: 1024 points 285 / 294 us, 4096 points 328 /
+//     264 us; 4000 x 3: 4096 points 223 / 232 us, 8192 points 335 / 240 us
+//   33 int16 frames, 1000 x 5: 6144 points 379 / 307 us, 8192 points 458 / 315 us; 4000 x 3: 12288 points 382 /
+//     355 us (41 FP16 frames 334 / 358 us), 16384 points 473 / 343 us
+//   33 float32 frames, 1000 x 5: 8192 points 332 / 358 us, 12288 points 436 / 368 us; 2500 x 5: 12288 points
+//     446 / 606 us, 20480 points 654 / 582 us
+bool copy_pays(bool cplx, int esz, uint32_t padded, uint64_t n_vox, uint64_t n_samples) {
+    if (padded <= 16) return n_vox >= std::max<uint64_t>(16384, 6 * n_samples);
+    if (cplx) return n_vox >= 2 * n_samples;
+    if (esz == 2) return n_vox >= std::max<uint64_t>(8192, 4 * n_samples);
+    return n_vox >= std::max<uint64_t>(12288, 8 * n_samples);
+}
+
 // interp < 0: a caller that runs neither the frame-lane nor the ensemble kernel; batch: a
 // persistent batch, which runs the frame-lane kernel but not the ensemble kernel; may_pad: the
 // caller can run a lane-voxel job on a copy of its channel data with padded frame rows; probe: the
@@ -477,7 +496,11 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
     const uintptr_t base = channel_on_device ? reinterpret_cast<uintptr_t>(channel) : 0;
     const bool rows_ok = n_frames > 8 && padded == n_frames && base % 32 == 0;
     const bool real8_ok = !cplx && n_frames > 16 && n_frames % 8 == 0 && base % ((8u * esz) % 32u == 0 ? 32 : 16) == 0;
-    const bool pad_ok = may_pad && n_frames > 8 && pad_fits(n_rx, n_samples, n_tx, padded, esz);
+    // Rows that the staged kernel can read as they are.  (host channel data is staged into fresh, aligned
+    // device buffers)
+    const bool vec_ok = n_frames % static_cast<uint32_t>(vf) == 0 && base % 8 == 0;
+    const bool pad_ok = may_pad && n_frames > 8 && pad_fits(n_rx, n_samples, n_tx, padded, esz) &&
+                        (vec_ok || copy_pays(cplx, esz, padded, n_vox, n_samples) || kind == MACH_B200_KERNEL_LANE_VOXEL);
     const bool chunks_ok = rows_ok || real8_ok || pad_ok;
     // Measured on B200 against the staged kernel: 12 complex64 frames x 3 transmits 619 -> 236 us, 12
     // float32 frames 464 -> 176 us, 9 int16 pairs 537 -> 237 us (all on padded copies), and against the
@@ -503,9 +526,6 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
         }
     }
     if (kind == MACH_B200_KERNEL_ENSEMBLE) kind = MACH_B200_KERNEL_AUTO;
-    // Host channel data is staged into fresh (aligned) device buffers.
-    const bool vec_ok =
-        n_frames % static_cast<uint32_t>(vf) == 0 && (!channel_on_device || reinterpret_cast<uintptr_t>(channel) % 8 == 0);
     if (kind == MACH_B200_KERNEL_AUTO) {
         kind = n_frames <= 8 || chunks_ok ? MACH_B200_KERNEL_LANE_VOXEL
                                           : (vec_ok ? MACH_B200_KERNEL_STAGED : MACH_B200_KERNEL_WARP);
