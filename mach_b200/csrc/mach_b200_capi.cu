@@ -810,7 +810,16 @@ struct DeviceBuffer {
         cudaError_t e = cudaGetDevice(&device);
         if (e == cudaSuccess) e = library_pool(device, &pool);
         if (e != cudaSuccess) return e;
-        return cudaMallocFromPoolAsync(&ptr, bytes ? bytes : 1, pool, st);
+        e = cudaMallocFromPoolAsync(&ptr, bytes ? bytes : 1, pool, st);
+        if (e == cudaErrorMemoryAllocation) {
+            // A pool that could not grow far enough keeps what it did get: back to the device with it
+            // (and with what it cached), for the caller's own allocations.
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            cudaThreadExchangeStreamCaptureMode(&mode);
+            cudaMemPoolTrimTo(pool, 0);
+            cudaThreadExchangeStreamCaptureMode(&mode);
+        }
+        return e;
     }
     ~DeviceBuffer() {
         if (ptr) cudaFreeAsync(ptr, stream);
