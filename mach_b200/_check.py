@@ -23,8 +23,12 @@ def is_contiguous(array: Any) -> bool:
 def ensure_contiguous(array: Any, *, warn: bool = True) -> Any:
     """Return a C-contiguous array, warning when a copy is made (src/mach/_check.py:25-41).  Views that
     torch conjugates or negates lazily are resolved."""
-    array = _dlpack.resolved(array)
-    if is_contiguous(array):
+    if _dlpack.is_torch(array):
+        if array.is_neg() or array.is_conj():
+            array = _dlpack.resolved(array)
+        if array.is_contiguous():
+            return array
+    elif is_contiguous(array):
         return array
     if warn:
         warnings.warn("array is not contiguous, rearranging will add latency", stacklevel=2)

@@ -122,22 +122,22 @@ def _from_capsule(obj: Any) -> ArrayView:
 _TORCH_DTYPE_NAMES: dict[Any, str] = {}  # torch dtype -> name, filled as dtypes are met
 
 
-def resolved(x: Any) -> Any:
-    """``x`` with its own values in memory: a torch view that is conjugated or negated by a flag only
-    (``x.conj()``, ``x.conj().imag``) is copied, anything else returned as it is."""
-    return x.resolve_conj().resolve_neg() if is_torch(x) else x
-
-
 def is_lazy(x: Any) -> bool:
     """Whether ``x`` is a torch view that is conjugated or negated by a flag only."""
     return is_torch(x) and (x.is_conj() or x.is_neg())
+
+
+def resolved(x: Any) -> Any:
+    """``x`` with its own values in memory: a torch view that is conjugated or negated by a flag only
+    (``x.conj()``, ``x.conj().imag``) is copied, anything else returned as it is."""
+    return x.resolve_conj().resolve_neg() if is_lazy(x) else x
 
 
 def _torch_view(t: Any) -> ArrayView:
     dtype = _TORCH_DTYPE_NAMES.get(t.dtype)
     if dtype is None:
         dtype = _TORCH_DTYPE_NAMES[t.dtype] = str(t.dtype).replace("torch.", "")
-    if t.is_conj() or t.is_neg():  # its memory does not hold its values (torch's own export refuses it too)
+    if t.is_neg() or (dtype[0] == "c" and t.is_conj()):  # its memory does not hold its values (torch's own export refuses it too)
         raise TypeError("lazily conjugated or negated tensor: call resolve_conj() / resolve_neg() first")
     cuda = t.is_cuda
     return ArrayView(t.data_ptr(), tuple(t.shape), t.stride(), dtype, t.element_size(), CUDA if cuda else CPU,

@@ -112,21 +112,23 @@ class Job:
         return int(self.scan_coords_m.shape[0]) * n_rx * n_tx * n_f
 
     def as_struct(self) -> _Job:
-        for name in ("channel", "rx_coords_m", "scan_coords_m", "arrivals", "out"):
-            t = getattr(self, name)
-            if not (t.is_cuda and t.is_contiguous()) or _dlpack.is_lazy(t):
+        channel, out = self.channel, self.out
+        for t in (channel, self.rx_coords_m, self.scan_coords_m, self.arrivals, out):
+            if not (t.is_cuda and t.is_contiguous()) or t.is_neg() or ((t is channel or t is out) and t.is_conj()):
+                name = next(n for n in ("channel", "rx_coords_m", "scan_coords_m", "arrivals", "out")
+                            if getattr(self, n) is t)
                 raise ValueError(f"Job.{name} must be a contiguous CUDA tensor (not lazily conjugated or negated)")
-        n_tx, n_rx, n_s, n_f = (int(d) for d in self.channel.shape[:4])
+        n_tx, n_rx, n_s, n_f = channel.shape[:4]
         j = _Job()
         j.storage = _cuda_impl.STORAGE_CODES[self.storage]
         j.interp_type = int(self.interp_type)
-        j.channel_data = self.channel.data_ptr()
+        j.channel_data = channel.data_ptr()
         j.rx_coords_m = self.rx_coords_m.data_ptr()
         j.scan_coords_m = self.scan_coords_m.data_ptr()
         j.tx_wave_arrivals_s = self.arrivals.data_ptr()
-        j.out = self.out.data_ptr()
+        j.out = out.data_ptr()
         j.n_tx, j.n_rx, j.n_samples, j.n_frames = n_tx, n_rx, n_s, n_f
-        j.n_scan = int(self.scan_coords_m.shape[0])
+        j.n_scan = self.scan_coords_m.shape[0]
         j.f_number, j.rx_start_s = float(self.f_number), float(self.rx_start_s)
         j.sampling_freq_hz, j.sound_speed_m_s = float(self.sampling_freq_hz), float(self.sound_speed_m_s)
         j.modulation_freq_hz, j.tukey_alpha = float(self.modulation_freq_hz), float(self.tukey_alpha)
@@ -140,8 +142,7 @@ class Job:
         grid = t.get("grid_shape")
         grid = self.grid_shape if grid is None else grid
         if grid:
-            for i, v in enumerate(grid):
-                j.grid_shape[i] = int(v)
+            j.grid_shape[:] = [int(v) for v in grid]
         kernel = t.get("kernel", 0)
         j.kernel = _cuda_impl.KERNELS[kernel] if isinstance(kernel, str) else int(kernel)
         j.tx_chunk = int(t.get("tx_chunk", 0))

@@ -135,6 +135,7 @@ struct SideStream {
     cudaStream_t stream = nullptr;
     cudaEvent_t event = nullptr;
     int priority = 0;
+    enum Use { kIdle, kBusy, kCaptured } left = kIdle;  // as the last run left it
 };
 constexpr int kMaxSideStreams = 24;  // per device, all batches and threads together
 
@@ -217,42 +218,47 @@ struct SideStreams {
         dev = d;
         int priority = 0;
         cudaStreamGetPriority(caller, &priority);
+        std::lock_guard<std::mutex> lock(d->side_mutex);
+        d->side_free.reserve(kMaxSideStreams);  // the way back allocates nothing
+        auto take_if = [&](auto usable) {
+            for (size_t i = 0; i < d->side_free.size() && static_cast<int>(taken.size()) < n;) {
+                if (d->side_free[i].priority == priority && usable(d->side_free[i])) {
+                    taken.push_back(d->side_free[i]);
+                    d->side_free.erase(d->side_free.begin() + static_cast<std::ptrdiff_t>(i));
+                } else {
+                    ++i;
+                }
+            }
+        };
+        take_if([](const SideStream& s) { return s.left == SideStream::kIdle; });
+        if (static_cast<int>(taken.size()) == n) return;
         // (queries and stream creation must not disturb a capture of this or another thread)
         cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
         cudaThreadExchangeStreamCaptureMode(&mode);
-        {
-            std::lock_guard<std::mutex> lock(d->side_mutex);
-            d->side_free.reserve(kMaxSideStreams);  // the way back allocates nothing
-            for (int pass = 0; pass < 2; ++pass) {  // idle streams and new ones, then busy ones
-                for (size_t i = 0; i < d->side_free.size() && static_cast<int>(taken.size()) < n;) {
-                    const SideStream s = d->side_free[i];
-                    cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
-                    const bool usable = s.priority == priority &&
-                                        cudaStreamIsCapturing(s.stream, &status) == cudaSuccess &&
-                                        status == cudaStreamCaptureStatusNone &&
-                                        (pass == 1 || cudaStreamQuery(s.stream) == cudaSuccess);
-                    if (!usable) {
-                        ++i;
-                        continue;
-                    }
-                    taken.push_back(s);
-                    d->side_free.erase(d->side_free.begin() + static_cast<std::ptrdiff_t>(i));
-                }
-                while (pass == 0 && static_cast<int>(taken.size()) < n && d->side_total < kMaxSideStreams) {
-                    SideStream s;
-                    s.priority = priority;
-                    if (cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, priority) != cudaSuccess) break;
-                    if (cudaEventCreateWithFlags(&s.event, cudaEventDisableTiming) != cudaSuccess) {
-                        cudaStreamDestroy(s.stream);
-                        break;
-                    }
-                    ++d->side_total;
-                    taken.push_back(s);
-                }
+        auto in_capture = [](const SideStream& s) {
+            cudaStreamCaptureStatus status = cudaStreamCaptureStatusActive;
+            return s.left == SideStream::kCaptured &&
+                   (cudaStreamIsCapturing(s.stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone);
+        };
+        take_if([&](const SideStream& s) { return !in_capture(s) && cudaStreamQuery(s.stream) == cudaSuccess; });
+        while (static_cast<int>(taken.size()) < n && d->side_total < kMaxSideStreams) {
+            SideStream s;
+            s.priority = priority;
+            if (cudaStreamCreateWithPriority(&s.stream, cudaStreamNonBlocking, priority) != cudaSuccess) break;
+            if (cudaEventCreateWithFlags(&s.event, cudaEventDisableTiming) != cudaSuccess) {
+                cudaStreamDestroy(s.stream);
+                break;
             }
+            ++d->side_total;
+            taken.push_back(s);
         }
+        take_if([&](const SideStream& s) { return !in_capture(s); });  // with earlier work still on them
         cudaThreadExchangeStreamCaptureMode(&mode);
         cudaGetLastError();  // a query's "not ready", or no room for a further stream: the run needs none
+    }
+    // Before the list gets them back: how the run that borrowed them leaves them.
+    void leave(SideStream::Use use) {
+        for (SideStream& s : taken) s.left = use;
     }
 };
 
@@ -1927,6 +1933,8 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
     std::vector<int> max_items(n_groups, 0);
     std::vector<double> points(n_groups, 0.0);
     std::vector<JobRange> written, read;
+    written.reserve(n_jobs);
+    read.reserve(size_t{4} * n_jobs);
     for (uint32_t i = 0; i < n_jobs; ++i) {
         const mach_b200_job& j = jobs[i];
         const uint64_t sums = j.n_scan * j.n_frames, samples = static_cast<uint64_t>(j.n_rx) * j.n_samples * j.n_frames;
@@ -1981,13 +1989,13 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
     }
 
     // ---- copies, counters, one persistent launch per group
+    cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
     if (n_jobs) {
         MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_jobs, b->h_jobs, sizeof(BatchJob) * parts.size(), cudaMemcpyHostToDevice, stream));
         MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_begin, b->h_begin, sizeof(int64_t) * parts.size(), cudaMemcpyHostToDevice, stream));
         MACH_B200_CUDA_TRY(cudaMemcpyAsync(b->d_hdr, b->h_hdr, sizeof(BatchHeader) * n_groups, cudaMemcpyHostToDevice, stream));
         MACH_B200_CUDA_TRY(cudaMemsetAsync(b->d_counters, 0, sizeof(unsigned long long) * n_groups, stream));
         // While capturing a graph the copies run at replay time, from the tables as they are then.
-        cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
         MACH_B200_CUDA_TRY(cudaStreamIsCapturing(stream, &capturing));
         if (capturing == cudaStreamCaptureStatusNone) {
             MACH_B200_CUDA_TRY(cudaEventRecord(b->copied, stream));
@@ -2005,6 +2013,7 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
     SideStreams sides;
     if (!in_order) sides.take(dev, stream, std::min<int>(mach_b200_batch::kSideStreams, static_cast<int>(order.size()) - 1));
     const int n_side = static_cast<int>(sides.taken.size());
+    sides.leave(capturing == cudaStreamCaptureStatusNone ? SideStream::kBusy : SideStream::kCaptured);
     if (n_side > 0) MACH_B200_CUDA_TRY(cudaEventRecord(sides.taken[0].event, stream));
     for (const SideStream& s : sides.taken) MACH_B200_CUDA_TRY(cudaStreamWaitEvent(s.stream, sides.taken[0].event, 0));
     cudaError_t launched = cudaSuccess;
@@ -2022,6 +2031,7 @@ int batch_run(mach_b200_batch* b, const mach_b200_job* jobs, uint32_t n_jobs, cu
     MACH_B200_CUDA_TRY(launched);
     if (!(flags & MACH_B200_FLAG_ASYNC)) {
         MACH_B200_CUDA_TRY(cudaStreamSynchronize(stream));
+        sides.leave(SideStream::kIdle);
         b->pending = false;
         if (any_waits) return check_status(dev, stream);
     }

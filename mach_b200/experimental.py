@@ -179,7 +179,7 @@ def _compound(channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out,
         raise ValueError("Output array `out` is not writable. Try using cupy or pytorch for the output array.")
     if not is_contiguous(out):
         raise ValueError("Output array `out` must be contiguous.")
-    if _dlpack.is_lazy(out):
+    if not fresh and _dlpack.is_lazy(out):
         raise ValueError("Output array `out` must not be a lazily conjugated or negated view.")
 
     rx = _dlpack.view(rx_coords_m)

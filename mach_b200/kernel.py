@@ -44,10 +44,10 @@ def _plain_tensors(channel_data: Any, rx_coords_m: Any, scan_coords_m: Any, tx_w
         return False
     tensor, f32 = torch.Tensor, torch.float32
     for x in (channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s):
-        if type(x) is not tensor or not x.is_cuda or not x.is_contiguous() or x.is_conj() or x.is_neg():
+        if type(x) is not tensor or not x.is_cuda or not x.is_contiguous() or x.is_neg():
             return False
     dtype = channel_data.dtype
-    if dtype is not f32 and dtype is not torch.complex64:
+    if dtype is not f32 and (dtype is not torch.complex64 or channel_data.is_conj()):
         return False
     if rx_coords_m.dtype is not f32 or scan_coords_m.dtype is not f32 or tx_wave_arrivals_s.dtype is not f32:
         return False
