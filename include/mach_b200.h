@@ -17,8 +17,13 @@
  * and fails with MACH_B200_ERR_CUDA.  The word is shared by all calls on a device, so a
  * timeout in an asynchronous call can be reported by the next synchronous call on any
  * stream of that device.  Temporary device buffers (host staging, work counters) come from
- * a memory pool of the library's own (at most 2 GiB of freed memory kept per device); the
- * process's default memory pool is never reconfigured.
+ * a memory pool of the library's own (at most 2 GiB of freed memory kept per device, and none of
+ * what a failed request got); the process's default memory pool is never reconfigured.  Scratch is
+ * taken by jobs with host buffers, by the ensemble kernel (a few counters), by frame counts above 8
+ * that are no whole chunks (a padded copy of the channel data, at most 1 GiB; without room for it
+ * the job runs on the rows as they are) and by power Doppler that is not fused (the frames' image;
+ * without room for it the ensemble kernel, if it takes the job).  Captured in a CUDA graph, such
+ * scratch becomes allocation nodes: the graph can be replayed, but not be a child graph.
  *
  * Layouts (C order):
  *   channel_data        [n_tx][n_rx][n_samples][n_frames] samples of `storage`
@@ -72,8 +77,10 @@ extern "C" {
                                          accurate than mach's FP32 delay; not bit-identical to mach) */
 #define MACH_B200_FLAG_POWER_DOPPLER 8u /* out is float32 [n_scan]: the power-Doppler image, the sum over
                                            frames of |beamformed value|^2 (the step after the beamformer
-                                           in mach's examples/doppler.py:252), fused into the kernel where
-                                           it can be; only the compound / _ex entry points take it */
+                                           in mach's examples/doppler.py:252).  Fused where the ensemble or
+                                           frame-lane kernel runs the job; else the frames' image is formed
+                                           in a temporary buffer and reduced.  Only the compound / _ex entry
+                                           points take it */
 #define MACH_B200_FLAG_PROBE_GRID 16u /* without a grid_shape, multi-frame jobs of device buffers look for the
                                          voxel grid on the device (one small kernel) and tile by it, as the
                                          single-transmit entry points do; never changes a sum */
@@ -111,9 +118,9 @@ typedef struct mach_b200_options {
                                 MACH_B200_TX_SPHERICAL: every (point, transmit) arrival is formed on the
                                 device from tx_params, by one kernel into a temporary [n_tx][n_scan]
                                 device array (tx_wave_arrivals_s may then be NULL) */
-    int32_t tile_fast;       /* lane-voxel kernels on a known grid: voxels a warp takes along the
-                                contiguous axis (1, 2, 4, 8 or 16; the rest of its 32 along the next
-                                axis), 0 = automatic */
+    int32_t tile_fast;       /* voxel-per-lane and frame-group kernels on a known grid: voxels a warp takes
+                                along the contiguous axis (1, 2, 4, 8 or 16; the rest of its voxels, 32 over
+                                the lanes per voxel, along the next axis), 0 = automatic */
     const double* tx_params; /* [n_tx][8]: origin xyz (m), unit direction (plane) or focus xyz (m)
                                 (spherical), time offset (s), unused.  The arrival is the distance of
                                 src/mach/wavefront.py:8-116 divided by the sound speed, plus the
@@ -122,12 +129,13 @@ typedef struct mach_b200_options {
                                 or 4, with runs of 16, 8 or 4 voxels; 0 = automatic */
     int32_t element_block;   /* voxel-per-lane kernels: elements per launch (the job runs as one launch
                                 per block of elements, accumulating), so that a launch's channel data
-                                stays in L2; 0 = automatic (blocks of about 80 MB of channel data for
-                                16-frame jobs above 126 MB), -1 or >= n_rx = one launch */
-    int32_t tile_order;      /* voxel-per-lane kernels on a known grid: 1 = CTAs take the tiles at the far
+                                stays in L2; 0 = automatic (blocks of about 80 MB of channel data above
+                                126 MB, for 16 frames and for real frames in chunks of 16), -1 or
+                                >= n_rx = one launch */
+    int32_t tile_order;      /* voxel-per-lane and frame-group kernels on a known grid: 1 = CTAs take the tiles at the far
                                 end of the contiguous axis first (the deepest first for a depth-fastest
                                 scan: widest aperture, most work, so a launch ends on light tiles),
-                                2 = grid order; 0 = automatic (1, except 16-frame jobs) */
+                                2 = grid order; 0 = automatic (1, except real frames in chunks of 16) */
 } mach_b200_options;
 
 /* Transmit models (mach_b200_options.tx_model). */

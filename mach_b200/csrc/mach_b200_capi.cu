@@ -509,7 +509,8 @@ Plan plan_launch(int storage, uint64_t n_vox, uint32_t n_frames, uint32_t n_tx, 
                         (vec_ok || copy_pays(cplx, esz, padded, n_vox, n_samples) || kind == MACH_B200_KERNEL_LANE_VOXEL);
     const bool chunks_ok = rows_ok || real8_ok || pad_ok;
     // Measured on B200 against the staged kernel: 12 complex64 frames x 3 transmits 619 -> 236 us, 12
-    // float32 frames 464 -> 176 us, 9 int16 pairs 537 -> 237 us (all on padded copies), and against the
+    // float32 frames 464 -> 176 us, 9 int16 pairs 537 -> 237 us (all on padded copies; 65536 points in random
+    // order, no grid: 1954 -> 607 us, 886 -> 280 us, 1038 -> 454 us), and against the
     // ensemble kernel: 200 complex64 frames 4.87 -> 3.67 ms, 64 int16 frames 757 -> 374 us (2-D) and
     // 64.9 -> 63.4 ms (3-D).  Float32 ensembles of 64 or more frames on a 3-D grid stay with the ensemble
     // kernel (60.7 ms against 75.6 ms; 2-D, 96 frames: 931 us against 797 us).
@@ -832,8 +833,6 @@ struct DeviceBuffer {
     }
 };
 
-// Launch transmits [0, a.n_tx) so that every launch's channel span stays below 2^31 samples
-// (32-bit offsets inside the kernels).  Later launches always accumulate.
 // Lane-voxel launches (which may run the elements in blocks, one launch each).
 bool lane_voxel_plan(const Plan& plan) {
     return !plan.staged && !plan.ensemble && !plan.frame_lane &&
@@ -883,6 +882,8 @@ bool element_block_staging(const Plan& plan, uint32_t n_rx) {
     return lane_voxel_plan(plan) && plan.lp.element_block > 0 && static_cast<uint32_t>(plan.lp.element_block) < n_rx;
 }
 
+// Launch transmits [0, a.n_tx) so that every launch's channel span stays below 2^31 samples
+// (32-bit offsets inside the kernels).  Later launches always accumulate.
 int dispatch_split(int storage, DasArgs a, int interp, const Plan& plan, cudaStream_t st) {
     const size_t esz = storage_bytes(storage);
     const int64_t per_tx = static_cast<int64_t>(a.n_rx) * a.row_stride;
@@ -1337,8 +1338,8 @@ mach_b200_options default_options(uint32_t flags) {
 // ---------------------------------------------------------------- power-Doppler epilogue
 //
 // out (float32 [n_scan]) (+)= sum over frames of |beamformed value|^2.  All-device jobs that
-// the ensemble kernel takes in one launch get the epilogue fused into the kernel (each frame
-// block adds its part atomically); every other job is beamformed into a temporary
+// the plan gives to the ensemble or frame-lane kernel in one launch get the epilogue fused into the
+// kernel (each frame block adds its part atomically); every other job is beamformed into a temporary
 // [n_scan][n_frames] image that one reduction kernel turns into the power image.
 
 int power_impl(int32_t storage, const void* channel_data, const float* rx_coords_m, const float* scan_coords_m,
@@ -1581,9 +1582,10 @@ int hilbert_impl(int32_t src_storage, const void* src, int32_t src_layout, int32
     }
     g.dst = dst;
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    // Contiguous destination columns of a length that its radices divide: the in-place kernel.  With
-    // several frames per sample the out-of-place kernel stays: it walks a group of up to 16
-    // columns column-fastest, so that its writes are contiguous too.
+    // Contiguous destination columns of a length that its radices divide: the in-place kernel, faster
+    // over lengths from 64 to 9216 (das_hilbert_cols.cu; 192 columns of 5120 or 5760 16-bit samples were 16
+    // and 6 % slower, nothing else).  With several frames per sample the out-of-place kernel stays: it
+    // walks a group of up to 16 columns column-fastest, so that its writes are contiguous too.
     HilbertColsArgs h{};
     const bool planned = F == 1 && hilbert_cols_plan(g.n, h);
     h.pair_vec = src_storage == kF32 && src_layout == MACH_B200_LAYOUT_ACQUISITION && n_cols % 2 == 0 &&

@@ -1,11 +1,13 @@
-"""Power-Doppler imaging fused with the beamformer.
+"""Power-Doppler imaging.
 
 mach's Doppler example beamforms an ensemble and then takes, per scan point, the sum over
 frames of the squared magnitude (``np.square(np.abs(result)).sum(axis=-1)``,
 examples/doppler.py:252; tests/compare/test_pymust.py:317-318).  :func:`power_doppler`
-returns that image directly.  When the ensemble kernel runs the job, the squares are summed
-inside the kernel as each frame block finishes, and the ``[n_points, n_frames]`` image is
-never written.
+returns that image directly.  Where the ensemble or frame-lane kernel runs the job (asked for, or
+float32 ensembles of 64 frames and more on a 3-D grid), the squares are summed inside the kernel as
+each frame block finishes, and the ``[n_points, n_frames]`` image is never written.  Every other job
+forms that image in a temporary buffer and reduces it, which is faster than the ensemble kernel;
+where the buffer does not fit, the ensemble kernel runs the job if it can.
 """
 
 from __future__ import annotations
@@ -40,9 +42,9 @@ def power_doppler(
     """Power-Doppler image ``sum_f |beamform(...)[:, f]|^2`` as float32 ``[n_points]``.
 
     Arguments are those of :func:`mach_b200.experimental.beamform`.  A GPU ``out`` is
-    accumulated into, a CPU ``out`` is overwritten.  The frame blocks of a scan point are
-    added in whatever order they finish, so the last bits can differ between runs
-    (relative 1e-7).
+    accumulated into, a CPU ``out`` is overwritten.  The fused kernels add the frame blocks of
+    a scan point in whatever order they finish, so there the last bits can differ between
+    runs (relative 1e-7).
     """
     return _compound(channel_data, rx_coords_m, scan_coords_m, tx_wave_arrivals_s, out, rx_start_s=rx_start_s,
                      sampling_freq_hz=sampling_freq_hz, f_number=f_number, sound_speed_m_s=sound_speed_m_s,
